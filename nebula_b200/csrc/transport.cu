@@ -316,9 +316,29 @@ __device__ __forceinline__ void store_resume(const Queue& q, uint32_t i, const F
 		(uint32_t)fr.type | ((uint32_t)fr.hop << 2) | ((uint32_t)fr.w.steps << 4)));
 }
 
-// Free flight(s) from the electron's current state: domain and energy cut,
-// free-path sampling, octree walk, move.  Flights in vacuum that hit nothing
-// end without an event and are repeated (the next one leaves the domain).
+// The checks a flight starts with: NaN state, domain, event budget, energy cut
+// (in that order; the flight is counted first).  False: the electron ends here.
+template<bool ADJ>
+__device__ __forceinline__ bool flight_begin(const StepParams& P, const DevGeometry& G, const Electron& p, int mat,
+	uint32_t& event, LocalCounters& lc, const float* dbar, const DevMaterial* mats)
+{
+	lc.add(CNT_FLIGHTS);
+	if (!(p.E == p.E) || !(p.pos.x == p.pos.x)) { lc.add(CNT_NAN); return false; }
+	if (!in_domain(G, p.pos.x, p.pos.y, p.pos.z))
+		return false;
+	if (event >= P.max_events) { lc.add(CNT_EVENT_BUDGET); return false; }
+	++event;
+	if (mat >= 0) {
+		const float barrier = (ADJ && dbar && mat < 2) ? fa(mats[mat].barrier, dbar[mat]) : mats[mat].barrier;
+		if (p.E < fa(barrier, P.energy_threshold))
+			return false;
+	}
+	return true;
+}
+
+// Free flight(s) of an electron whose flight_begin passed: free-path sampling,
+// octree walk, move.  Flights in vacuum that hit nothing end without an event
+// and are repeated (the next one leaves the domain).
 // Returns the queue of the event the flight ends in, -1 when the electron is
 // terminated, or EV_WALK when the walk reached the run's per-iteration cell
 // budget (`fr` then holds where it stands).  With `resume` non-null, the
@@ -336,6 +356,7 @@ __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& r
 		load_resume(*resume, resume_i, fr);
 		lc.add(CNT_RESUMED);
 	}
+	bool begun = true;
 	for (int hop = resume ? fr.hop : 0; hop < 4; ++hop) {
 		int type = 0;
 		float dist;
@@ -344,6 +365,7 @@ __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& r
 		WalkState w;
 		if (resume) {
 			resume = nullptr;
+			begun = false;
 			type = fr.type;
 			dist = fr.dist;
 			w = fr.w;
@@ -356,18 +378,12 @@ __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& r
 				}
 			}
 		} else {
-			lc.add(CNT_FLIGHTS);
-			if (!(p.E == p.E) || !(p.pos.x == p.pos.x)) { lc.add(CNT_NAN); return -1; }
-			if (!in_domain(G, p.pos.x, p.pos.y, p.pos.z))
+			if (!begun && !flight_begin<ADJ>(P, G, p, mat, event, lc, dbar, mats))
 				return -1;
-			if (event >= P.max_events) { lc.add(CNT_EVENT_BUDGET); return -1; }
-			++event;
+			begun = false;
 			dist = G.max_extent;
 			if (mat >= 0) {
 				m = mats + mat;
-				const float barrier = (ADJ && dbar && mat < 2) ? fa(m->barrier, dbar[mat]) : m->barrier;
-				if (p.E < fa(barrier, P.energy_threshold))
-					return -1;
 				PhiloxStream r;
 				r.init(rv.key, event, 0u, stream_tag, lineage);
 				const float pe = sample_path(m->el_imfp, m->el_scale, p.E, r, mu_el);
@@ -563,7 +579,7 @@ __device__ __forceinline__ void deposit(const StepParams& P, bool scat, const El
 
 template<bool ADJ, bool BATCH, bool DEP = false, uint32_t PHC = 0u>
 __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchParams& B, uint32_t it, LocalCounters& lc,
-	const DevMaterial* mats, float* s_lane = nullptr, const DevGeometry* s_geoms = nullptr,
+	const DevMaterial* mats, uint8_t* s_rank, float* s_lane = nullptr, const DevGeometry* s_geoms = nullptr,
 	const DevJob* s_jobs = nullptr)
 {
 	// physics selection bits: a compile-time constant in the instantiations
@@ -781,6 +797,83 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 				lc.add(CNT_TERMINATED);
 			}
 		}
+
+		// The checks the electron's own next flight starts with (a continued
+		// walk is past them).
+		bool flying = status == ST_RUNNING;
+		if (flying && kind != EV_WALK)
+			flying = flight_begin<ADJ>(P, *rv.geom, p, mat, event, lc, wshift ? dbar : nullptr, mats);
+		if (kind >= 0 && status != ST_DETECTED && !flying)
+			lc.add(CNT_TERMINATED);
+
+		// Half of the electrons end at the energy cut right after an inelastic
+		// event, and half of the events leave a secondary: a lane whose electron
+		// ended flies a secondary in its place (its own, else one of another
+		// lane's), in this iteration and without a trip through the flight
+		// queue.  Lanes past the end of the index space take none, so the
+		// population bound stays what it is.
+		const unsigned spawned = __ballot_sync(0xFFFFFFFFu, spawn);
+		if (spawned) {
+			bool take = spawn && !flying;
+			if (take)
+				spawn = false;
+			const unsigned donors = __ballot_sync(0xFFFFFFFFu, spawn);
+			const unsigned idle = __ballot_sync(0xFFFFFFFFu, kind >= 0 && !flying && !take);
+			const int moved = min(__popc(donors), __popc(idle));
+			uint32_t take_tag = tag;
+			int src = (int)lane;
+			if (moved) {
+				// donors write their lane at their rank, idle lanes read it at theirs
+				const int rank = __popc((spawn ? donors : idle) & lanemask_lt());
+				if (spawn && rank < moved) {
+					s_rank[rank] = (uint8_t)lane;
+					spawn = false;
+				}
+				__syncwarp();
+				if (kind >= 0 && !flying && !take && rank < moved) {
+					src = s_rank[rank];
+					take = true;
+				}
+				__syncwarp();
+				se.pos.x = __shfl_sync(0xFFFFFFFFu, p.pos.x, src);
+				se.pos.y = __shfl_sync(0xFFFFFFFFu, p.pos.y, src);
+				se.pos.z = __shfl_sync(0xFFFFFFFFu, p.pos.z, src);
+				se.dir.x = __shfl_sync(0xFFFFFFFFu, se.dir.x, src);
+				se.dir.y = __shfl_sync(0xFFFFFFFFu, se.dir.y, src);
+				se.dir.z = __shfl_sync(0xFFFFFFFFu, se.dir.z, src);
+				se.E = __shfl_sync(0xFFFFFFFFu, se.E, src);
+				se_lineage = __shfl_sync(0xFFFFFFFFu, se_lineage, src);
+				mat = __shfl_sync(0xFFFFFFFFu, mat, src);
+				take_tag = __shfl_sync(0xFFFFFFFFu, tag, src);
+				if (ADJ) {
+#pragma unroll
+					for (int k = 0; k < 6; ++k) sc[k] = __shfl_sync(0xFFFFFFFFu, sc[k], src);
+				}
+			}
+			if (take) {
+				p = se;
+				lineage = se_lineage;
+				last_tri = -1;
+				event = 0u;
+				tag = take_tag;
+				if (BATCH) {
+					job = tag >> 24;
+					stream_tag = tag & 0xFFFFFFu;
+					const DevJob& J = s_jobs[job];
+					rv.geom = s_geoms + J.geom;
+					rv.key = J.key;
+				} else {
+					stream_tag = tag;
+				}
+				if (wshift) {
+					dbar[0] = fm(P.wstep, wsign(rv.key, stream_tag, 0));
+					dbar[1] = fm(P.wstep, wsign(rv.key, stream_tag, 1));
+				}
+				flying = flight_begin<ADJ>(P, *rv.geom, p, mat, event, lc, wshift ? dbar : nullptr, mats);
+				if (!flying)
+					lc.add(CNT_TERMINATED);
+			}
+		}
 		// The flight queue's counter hands out the tickets: the first
 		// se_budget secondaries are queued, later ones go to the spill ring
 		// (their slots stay unwritten; the next iteration reads at most
@@ -813,10 +906,10 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 
 		// next free flight (or the rest of a walk cut short last iteration)
 		int qtype = -1;
-		if (status == ST_RUNNING)
+		if (flying)
 			qtype = free_flight<ADJ>(P, rv, p, mat, last_tri, event, stream_tag, lineage, sc, lc,
 				wshift ? dbar : nullptr, fr, kind == EV_WALK ? &qin[EV_WALK] : nullptr, qi, mats);
-		if (kind >= 0 && status != ST_DETECTED && qtype < 0)
+		if (flying && qtype < 0)
 			lc.add(CNT_TERMINATED);
 		{
 			// the warp's next chunk is claimed (lane 5) together with the
@@ -896,6 +989,7 @@ __global__ void __launch_bounds__(256, NBL_STEP_MIN_BLOCKS) k_step(const __grid_
 {
 	__shared__ uint32_t s_counters[N_COUNTERS];
 	__shared__ float s_lane[DEP ? 256 : 1];
+	__shared__ uint8_t s_rank[256];
 	for (int k = threadIdx.x; k < N_COUNTERS; k += blockDim.x)
 		s_counters[k] = 0u;
 	__syncthreads();
@@ -904,7 +998,7 @@ __global__ void __launch_bounds__(256, NBL_STEP_MIN_BLOCKS) k_step(const __grid_
 	// materials read from global memory: staged in shared memory as the
 	// batched kernel stages them, this kernel measured slower (-0.4 % on the
 	// grating scan, -1.5 % on the 1.2 M-triangle mesh)
-	step_iteration<ADJ, false, DEP, PHC>(P, none, it, lc, P.mats, s_lane);
+	step_iteration<ADJ, false, DEP, PHC>(P, none, it, lc, P.mats, s_rank + (threadIdx.x & ~31u), s_lane);
 	flush_counters(P, s_counters);
 }
 
@@ -955,6 +1049,7 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 	// its chain of dependent loads, and shared loads are the shorter ones
 	__shared__ DevGeometry s_geoms[NBL_BATCH_MAX_GEOMS];
 	__shared__ DevJob s_jobs[NBL_BATCH_MAX_JOBS];
+	__shared__ uint8_t s_rank[512];
 	for (int k = threadIdx.x; k < N_COUNTERS; k += blockDim.x)
 		s_counters[k] = 0u;
 	for (int k = threadIdx.x; k < B.n_geoms; k += blockDim.x)
@@ -966,7 +1061,7 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 	LocalCounters lc{ s_counters };
 	uint32_t it = 0;
 	for (; it < B.max_iterations; ++it) {
-		if (!step_iteration<ADJ, true, false, PHC>(P, B, it, lc, s_mats, nullptr, s_geoms, s_jobs))
+		if (!step_iteration<ADJ, true, false, PHC>(P, B, it, lc, s_mats, s_rank + (threadIdx.x & ~31u), nullptr, s_geoms, s_jobs))
 			break;
 		if (!grid_barrier(B))
 			break;
