@@ -849,6 +849,10 @@ nbl_status nbl_sim_create(const nbl_geometry* g, nbl_material* const* materials,
 		// refill target; the secondary budget keeps the population below it
 		require((uint64_t)cap * 8 < (1ull << 30), "capacity too large");
 		sp.qcap = 8 * cap;
+		// secondaries are parked from 6x on: since ended lanes fly most of
+		// them, populations peak at 3.2 (slab, 1 keV) to 4.7 times the target
+		// (grating), at 7 to 8 times in pools below a hundred
+		sp.pop_bound = 6 * cap;
 		// refill at most 1/16 of the target per iteration, so the population
 		// ramps up while the cascades of the first primaries develop
 		sp.ramp = std::max<uint32_t>(cap / 16, 256);
