@@ -68,7 +68,8 @@ struct Electron {
 	float E;
 };
 
-template<class R> __device__ __forceinline__ float draw_phi(R& rng) { return fm(2.0f * NBL_PI, rng.unit()); }
+// azimuth from a uniform draw
+__device__ __forceinline__ float draw_phi(float u) { return fm(2.0f * NBL_PI, u); }
 
 // make_unit_vec (vector_math.h:194-206)
 __device__ __forceinline__ V3 make_unit_vec(float cos_theta, float phi)
@@ -79,11 +80,10 @@ __device__ __forceinline__ V3 make_unit_vec(float cos_theta, float phi)
 	const float st = __fsqrt_rn(fs(1.0f, fm(cos_theta, cos_theta)));
 	return v3(fm(st, cp), fm(st, sp), cos_theta);
 }
-template<class R> __device__ __forceinline__ V3 uniform_vector(R& rng)
+// isotropic direction from two uniform draws: the azimuth's, then the polar cosine's
+__device__ __forceinline__ V3 uniform_vector(float u_phi, float u_cos)
 {
-	const float phi = draw_phi(rng);
-	const float ct = fs(fm(2.0f, rng.unit()), 1.0f);
-	return make_unit_vec(ct, phi);
+	return make_unit_vec(fs(fm(2.0f, u_cos), 1.0f), draw_phi(u_phi));
 }
 // make_normal_vec (vector_math.h:171-186)
 __device__ __forceinline__ V3 make_normal_vec(V3 dir, float phi)
@@ -104,138 +104,169 @@ __device__ __forceinline__ float imfp_at(const DevTable& imfp_tab, float scale, 
 }
 
 // One exponential free path: -tau * log(U), tau = 1 / (scale * exp(table(log E)))
-template<class R> __device__ __forceinline__ float sample_path(const DevTable& imfp_tab, float scale, float E, R& rng, float& mu)
+__device__ __forceinline__ float sample_path(const DevTable& imfp_tab, float scale, float E, float u, float& mu)
 {
 	mu = imfp_at(imfp_tab, scale, E);
 	const float tau = fdf(1.0f, mu);
-	return fm(-tau, __logf(rng.unit()));
+	return fm(-tau, __logf(u));
 }
 
-// Elastic event (elastic.h:67-115), acoustic-phonon and atomic-recoil loss
-// as selected.
-template<class R> __device__ __forceinline__ void elastic_event(const DevMaterial& m, Electron& p, R& rng,
-	uint32_t ph = PH_DEFAULT)
+// Reduced energy of the electron a plasmon decays into, trial draws U1, U2,
+// and the probability to accept it.
+struct PlasmonDecay { float alpha, d1, d2, lower; };
+__device__ __forceinline__ float decay_trial(const PlasmonDecay& k, float U1, float U2, float& acc)
 {
-	const float x = __logf(p.E);
-	const float y = rng.unit();
-	const float cos_theta = clampf(table2_get(m.el_icdf, x, y), -1.0f, 1.0f);
-	const float sin_theta = __fsqrt_rn(fs(1.0f, fm(cos_theta, cos_theta)));
-	p.dir = vnormalised(p.dir);
-	const V3 normal_dir = vnormalised(make_normal_vec(p.dir, draw_phi(rng)));
-	p.dir = vadd(vmul(p.dir, cos_theta), vmul(normal_dir, sin_theta));
-	if (p.E < 200.0f) {
-		if (ph & PH_PHONON)
-			p.E = fs(p.E, smin(50e-3f, m.phonon_loss));
-	} else if (ph & PH_RECOIL) {
-		p.E = fs(p.E, fm(fm(m.recoil_const, fs(1.0f, cos_theta)), p.E));
-	}
+	const float x = (U1 < k.alpha) ? __fsqrt_rn(fa(fm(k.d2, U2), fm(k.lower, k.lower))) : fa(fm(k.d1, U2), k.lower);
+	acc = fdf(__fsqrt_rn(fa(fm(x, x), x)), fa(x, 0.5f));
+	return x;
 }
 
-// Inelastic event (full_penn.h:62-288).  Returns true and fills `se` when a
+// Scatter event of one electron: elastic (elastic.h:67-115; acoustic-phonon
+// and atomic-recoil loss as selected) or inelastic of the Full-Penn model
+// (full_penn.h:62-288).  `u`: the event's draws 0..3; `rng` gives the later
+// ones and is told how many were taken.  Returns true and fills `se` when a
 // secondary electron is created.  The plasmon-decay rejection loop is capped
 // at 64 trials (the last trial is kept); the reference loop is unbounded but
 // its acceptance rate is above one half.
-template<class R> __device__ __forceinline__ bool penn_event(const DevMaterial& m, Electron& p, Electron& se, R& rng,
-	uint32_t ph)
+// The two kinds share what they have in common -- the first table lookup, the
+// normalised direction, the random normal to it -- and so do the branches of
+// the inelastic event: the step kernel waits for instruction fetches, and one
+// copy of each of these is fetched once.
+template<class R> __device__ __forceinline__ bool scatter_event(bool elastic, const DevMaterial& m, Electron& p,
+	Electron& se, const float (&u)[4], R& rng, uint32_t ph)
 {
-	float omega;
-	{
-		const float x = __logf(p.E);
-		const float y = rng.unit();
-		omega = __expf(table2_get(m.in_omega, x, y));
-	}
-	float binding;
-	{
-		const float x = __logf(p.E);
-		const float y = __logf(fdf(omega, p.E));
-		const float z = rng.unit();
-		binding = table3_rounddown(m.in_binding, x, y, z);
-	}
+	const float x = __logf(p.E);
+	const float t0 = table2_get(elastic ? m.el_icdf : m.in_omega, x, u[0]);
 	p.dir = vnormalised(p.dir);
-	if (binding <= 0.0f) {
-		if (omega > m.band_gap) {
-			float q;
-			{
-				const float x = __logf(p.E);
-				const float y = fdf(omega, p.E);
-				const float z = rng.unit();
-				q = table3_get(m.in_q, x, y, z);
-			}
-			const V3 prim_normal_dir = vnormalised(make_normal_vec(p.dir, draw_phi(rng)));
-			V3 q_dir, q_normal_dir;
-			{
-				const float c = clampf(fdf(fa(omega, fm(q, q)), fm(fm(2.0f, __fsqrt_rn(p.E)), q)), -1.0f, 1.0f);
-				const float s = __fsqrt_rn(fs(1.0f, fm(c, c)));
-				q_dir = vnormalised(vadd(vmul(p.dir, c), vmul(prim_normal_dir, s)));
-				q_normal_dir = vnormalised(make_normal_vec(q_dir, draw_phi(rng)));
-			}
-			const float c2 = clampf(fdf(fs(fs(fm(2.0f, p.E), omega), fm(q, q)),
-				fm(2.0f, __fsqrt_rn(fm(p.E, fs(p.E, omega))))), -1.0f, 1.0f);
-			const float s2 = __fsqrt_rn(fs(1.0f, fm(c2, c2)));
-			p.E = fs(p.E, omega);
-			p.dir = vadd(vmul(p.dir, c2), vmul(prim_normal_dir, s2));
-			if (!(ph & PH_GEN_SE))
-				return false;
-
-			se.pos = p.pos;
-			const float k_fermi = __fsqrt_rn(m.fermi);
-			const float k_fermi_omega = __fsqrt_rn(fa(m.fermi, omega));
-			if (q < fs(k_fermi_omega, k_fermi)) {
-				// plasmon decay
-				const float f = fdf(m.fermi, omega);
-				float x;
-				if (f < 0.1f) {
-					const float U = cbrtf(rng.unit());
-					x = fm(fm(f, U), U);
-				} else {
-					const float lower = smax(0.0f, fs(f, 1.0f));
-					const float upper = f;
-					const float d1 = fs(upper, lower);
-					const float d2 = fs(fm(upper, upper), fm(lower, lower));
-					const float alpha = fdf(d2, fa(d1, d2));
-					int trial = 0;
-					for (;;) {
-						const float U1 = rng.unit();
-						const float U2 = rng.unit();
-						x = (U1 < alpha) ? __fsqrt_rn(fa(fm(d2, U2), fm(lower, lower))) : fa(fm(d1, U2), lower);
-						const float acc = fdf(__fsqrt_rn(fa(fm(x, x), x)), fa(x, 0.5f));
-						if (!(rng.unit() > acc) || ++trial >= 64)
-							break;
-					}
-				}
-				se.E = fa(fm(x, omega), omega);
-				se.dir = uniform_vector(rng);
-			} else if (q < fa(k_fermi_omega, k_fermi)) {
-				// single excitation from the Fermi sphere
-				const float ki_parr = fdf(fs(omega, fm(q, q)), fm(2.0f, q));
-				const float kf_parr = fa(ki_parr, q);
-				const float ki_perp_min_sq = smax(0.0f, fs(m.fermi, fm(kf_parr, kf_parr)));
-				const float ki_perp_max_sq = fs(m.fermi, fm(ki_parr, ki_parr));
-				const float ki_perp_sq = smax(0.0f, fa(ki_perp_min_sq, fm(fs(ki_perp_max_sq, ki_perp_min_sq), rng.unit())));
-				const V3 ki = vadd(smul(ki_parr, q_dir), smul(__fsqrt_rn(ki_perp_sq), q_normal_dir));
-				se.E = fa(vmag2(ki), omega);
-				se.dir = vadd(ki, smul(q, q_dir));
-			} else {
-				return false;
-			}
-			return true;
-		} else {
+	float omega = 0.0f, binding = 0.0f, u_phi = u[1];
+	bool inner = false;
+	rng.n = 2;
+	if (!elastic) {
+		omega = __expf(t0);
+		binding = table3_rounddown(m.in_binding, x, __logf(fdf(omega, p.E)), u[1]);
+		inner = !(binding <= 0.0f);
+		if (!inner && !(omega > m.band_gap)) {
 			p.E = fs(p.E, omega);
 			return false;
 		}
+		u_phi = inner ? u[2] : u[3];
+	}
+	const V3 normal_dir = vnormalised(make_normal_vec(p.dir, draw_phi(u_phi)));
+	if (elastic) {
+		const float cos_theta = clampf(t0, -1.0f, 1.0f);
+		const float sin_theta = __fsqrt_rn(fs(1.0f, fm(cos_theta, cos_theta)));
+		p.dir = vadd(vmul(p.dir, cos_theta), vmul(normal_dir, sin_theta));
+		if (p.E < 200.0f) {
+			if (ph & PH_PHONON)
+				p.E = fs(p.E, smin(50e-3f, m.phonon_loss));
+		} else if (ph & PH_RECOIL) {
+			p.E = fs(p.E, fm(fm(m.recoil_const, fs(1.0f, cos_theta)), p.E));
+		}
+		return false;
+	}
+	float w[4];                               // draws 4..7
+	rng.block(1, w);
+	rng.n = 5;
+	se.pos = p.pos;
+	// draws of an isotropic direction, and the energy scale of a decay
+	float v_phi = u[3], v_cos = w[0], decay = 0.0f;
+	if (!inner) {
+		const float q = table3_get(m.in_q, x, fdf(omega, p.E), u[2]);
+		V3 q_dir;
+		{
+			const float c = clampf(fdf(fa(omega, fm(q, q)), fm(fm(2.0f, __fsqrt_rn(p.E)), q)), -1.0f, 1.0f);
+			const float s = __fsqrt_rn(fs(1.0f, fm(c, c)));
+			q_dir = vnormalised(vadd(vmul(p.dir, c), vmul(normal_dir, s)));
+		}
+		const float c2 = clampf(fdf(fs(fs(fm(2.0f, p.E), omega), fm(q, q)),
+			fm(2.0f, __fsqrt_rn(fm(p.E, fs(p.E, omega))))), -1.0f, 1.0f);
+		const float s2 = __fsqrt_rn(fs(1.0f, fm(c2, c2)));
+		p.E = fs(p.E, omega);
+		p.dir = vadd(vmul(p.dir, c2), vmul(normal_dir, s2));
+		if (!(ph & PH_GEN_SE))
+			return false;
+
+		const float k_fermi = __fsqrt_rn(m.fermi);
+		const float k_fermi_omega = __fsqrt_rn(fa(m.fermi, omega));
+		if (!(q < fs(k_fermi_omega, k_fermi))) {
+			if (!(q < fa(k_fermi_omega, k_fermi)))
+				return false;
+			// single excitation from the Fermi sphere (draw 4 gives the normal to q)
+			const V3 q_normal_dir = vnormalised(make_normal_vec(q_dir, draw_phi(w[0])));
+			const float ki_parr = fdf(fs(omega, fm(q, q)), fm(2.0f, q));
+			const float kf_parr = fa(ki_parr, q);
+			const float ki_perp_min_sq = smax(0.0f, fs(m.fermi, fm(kf_parr, kf_parr)));
+			const float ki_perp_max_sq = fs(m.fermi, fm(ki_parr, ki_parr));
+			const float ki_perp_sq = smax(0.0f, fa(ki_perp_min_sq, fm(fs(ki_perp_max_sq, ki_perp_min_sq), w[1])));
+			const V3 ki = vadd(smul(ki_parr, q_dir), smul(__fsqrt_rn(ki_perp_sq), q_normal_dir));
+			se.E = fa(vmag2(ki), omega);
+			se.dir = vadd(ki, smul(q, q_dir));
+			rng.n = 6;
+			return true;
+		}
+		// plasmon decay
+		const float f = fdf(m.fermi, omega);
+		if (f < 0.1f) {
+			const float U = cbrtf(w[1]);
+			decay = fm(fm(f, U), U);
+			v_phi = w[2]; v_cos = w[3];
+			rng.n = 8;
+		} else {
+			PlasmonDecay k;
+			k.lower = smax(0.0f, fs(f, 1.0f));
+			k.d1 = fs(f, k.lower);
+			k.d2 = fs(fm(f, f), fm(k.lower, k.lower));
+			k.alpha = fdf(k.d2, fa(k.d1, k.d2));
+			float acc;
+			decay = decay_trial(k, w[1], w[2], acc);
+			// one draw per pass from draw 8 on: three for each further trial
+			// (step 0..2), two for the direction (step 3, 4)
+			int trial = 1, step = w[3] > acc ? 0 : 3;
+			uint32_t n = 8;
+			float U1 = 0.0f;
+			for (;;) {
+				if ((n & 3u) == 0u)
+					rng.block(n >> 2, w);
+				const uint32_t j = n & 3u;
+				const float r = j == 0u ? w[0] : j == 1u ? w[1] : j == 2u ? w[2] : w[3];
+				++n;
+				if (step == 0) {
+					U1 = r;
+				} else if (step == 1) {
+					decay = decay_trial(k, U1, r, acc);
+				} else if (step == 2) {
+					if (r > acc && ++trial < 64) {
+						step = 0;
+						continue;
+					}
+				} else if (step == 3) {
+					v_phi = r;
+				} else {
+					v_cos = r;
+					break;
+				}
+				++step;
+			}
+			rng.n = n;
+		}
+		decay = fa(fm(decay, omega), omega);
+	}
+	const V3 v = uniform_vector(v_phi, v_cos);
+	if (!inner) {
+		se.E = decay;
+		se.dir = v;
+		return true;
 	}
 	// inner-shell ionisation (Ivanchenko angles)
-	const V3 normal_dir = vnormalised(make_normal_vec(p.dir, draw_phi(rng)));
 	const float K = fa(fs(p.E, m.fermi), fm(2.0f, binding));
 	const float dK = fa(binding, omega);
 	const float cos_theta = __fsqrt_rn(fdf(dK, K));
 	const float sin_theta = __fsqrt_rn(fs(1.0f, clampf(fm(cos_theta, cos_theta), 0.0f, 1.0f)));
 	V3 sdir = vadd(vmul(p.dir, cos_theta), vmul(normal_dir, sin_theta));
 	sdir = vnormalised(sdir);
-	sdir = vadd(sdir, smul(__fsqrt_rn(fdf(binding, dK)), uniform_vector(rng)));
+	sdir = vadd(sdir, smul(__fsqrt_rn(fdf(binding, dK)), v));
 	sdir = vnormalised(sdir);
 	se.E = fs(fa(m.fermi, omega), binding);
-	se.pos = p.pos;
 	se.dir = sdir;
 	p.E = fs(p.E, omega);
 	p.dir = vsub(p.dir, smul(cos_theta, sdir));
@@ -248,21 +279,12 @@ template<class R> __device__ __forceinline__ bool penn_event(const DevMaterial& 
 // limits, Ivanchenko angles for the secondary.  The two logarithms and the
 // expm1 of the omega draw take arguments close to 1 and 0, so they use the
 // accurate library functions rather than the SFU forms.
-template<class R> __device__ __forceinline__ bool kieft_event(const DevMaterial& m, Electron& p, Electron& se, R& rng,
-	uint32_t ph)
+template<class R> __device__ __forceinline__ bool kieft_event(const DevMaterial& m, Electron& p, Electron& se,
+	const float (&u)[4], R& rng, uint32_t ph)
 {
-	float omega0;
-	{
-		const float x = __logf(p.E);
-		const float y = rng.unit();
-		omega0 = __expf(table2_get(m.in_omega, x, y));
-	}
-	float binding;
-	{
-		const float x = __logf(omega0);
-		const float y = rng.unit();
-		binding = table2_rounddown(m.in_binding, x, y);
-	}
+	const float omega0 = __expf(table2_get(m.in_omega, __logf(p.E), u[0]));
+	float binding = table2_rounddown(m.in_binding, __logf(omega0), u[1]);
+	rng.n = 3;
 	float omega;
 	{
 		const float omega_max = fm(0.5f, fs(fa(p.E, omega0), m.fermi));
@@ -272,7 +294,7 @@ template<class R> __device__ __forceinline__ bool kieft_event(const DevMaterial&
 			omega_min = fm(0.5f, fs(fa(p.E, omega0), __fsqrt_rn(fm(p.E, fs(p.E, fm(2.0f, omega0))))));
 			w0 = omega0;
 		}
-		const float U = rng.unit();
+		const float U = u[2];
 		if ((w0 > 0.0f) && (omega_min > w0) && (omega_min < omega_max)) {
 			const float f_min = fm(fdf(1.0f, w0), logf(fdf(fs(omega_min, w0), omega_min)));
 			const float f_max = fm(fdf(1.0f, w0), logf(fdf(fs(omega_max, w0), omega_max)));
@@ -294,15 +316,19 @@ template<class R> __device__ __forceinline__ bool kieft_event(const DevMaterial&
 	}
 	binding = smax(0.0f, binding);
 	p.dir = vnormalised(p.dir);
-	const V3 normal_dir = vnormalised(make_normal_vec(p.dir, draw_phi(rng)));
+	const V3 normal_dir = vnormalised(make_normal_vec(p.dir, draw_phi(u[3])));
+	rng.n = 4;
 	const float K = fa(fs(p.E, m.fermi), fm(2.0f, binding));
 	const float dK = fa(binding, omega);
 	const float cos_theta = __fsqrt_rn(fdf(dK, K));
 	const float sin_theta = __fsqrt_rn(fs(1.0f, clampf(fm(cos_theta, cos_theta), 0.0f, 1.0f)));
 	V3 sdir = vadd(vmul(p.dir, cos_theta), vmul(normal_dir, sin_theta));
 	if (ph & PH_INST_MOM) {
+		float w[4];                           // draws 4..7
+		rng.block(1, w);
+		rng.n = 6;
 		sdir = vnormalised(sdir);
-		sdir = vadd(sdir, smul(__fsqrt_rn(fdf(binding, dK)), uniform_vector(rng)));
+		sdir = vadd(sdir, smul(__fsqrt_rn(fdf(binding, dK)), uniform_vector(w[0], w[1])));
 	}
 	sdir = vnormalised(sdir);
 	se.E = fs(fa(m.fermi, omega), binding);
@@ -314,26 +340,16 @@ template<class R> __device__ __forceinline__ bool kieft_event(const DevMaterial&
 	return (ph & PH_GEN_SE) != 0;
 }
 
-// Inelastic event of the selected model.  Returns true and fills `se` when a
-// secondary electron is created.
-template<class R> __device__ __forceinline__ bool inelastic_event(const DevMaterial& m, Electron& p, Electron& se, R& rng,
-	uint32_t ph = PH_DEFAULT)
-{
-	if (ph & PH_KIEFT)
-		return kieft_event(m, p, se, rng, ph);
-	return penn_event(m, p, se, rng, ph);
-}
-
 enum : int { ST_RUNNING = 0, ST_DETECTED = 1, ST_TERMINATED = 2 };
 
 // Boundary crossing (boundary_intersect.h:38-155) with quantum transmission,
 // refraction and the Kieft-Bosch empirical absorption as selected.  `score`
 // (optional) receives d log P(outcome) / d barrier_out and d / d barrier_in
-// for the adjoint.
+// for the adjoint.  `u`: the event's draws 0..3; `n` receives how many were taken.
 struct BoundaryScore { float d_in, d_out; int mat_in, mat_out; };
 
-template<class R> __device__ __forceinline__ int boundary_event(const DevTriangle& T, const DevMaterial* __restrict__ mats,
-	Electron& p, int& material, R& rng, BoundaryScore* score = nullptr, uint32_t ph = PH_DEFAULT,
+__device__ __forceinline__ int boundary_event(const DevTriangle& T, const DevMaterial* __restrict__ mats,
+	Electron& p, int& material, const float (&u)[4], uint32_t& n_used, BoundaryScore* score, uint32_t ph,
 	const float* dbar = nullptr)
 {
 	const V3 nd = vnormalised(p.dir);
@@ -361,7 +377,8 @@ template<class R> __device__ __forceinline__ int boundary_event(const DevTriangl
 		const float s = __fsqrt_rn(fa(1.0f, fdf(dU, Ec2)));
 		const bool qt = (ph & PH_QT) != 0;
 		const float Tr = qt ? fdf(fm(4.0f, s), fm(fa(1.0f, s), fa(1.0f, s))) : 1.0f;
-		const bool transmit = rng.unit() < Tr;
+		const bool transmit = u[0] < Tr;
+		n_used = 1;
 		if (score && qt) {
 			// T(s) = 4s/(1+s)^2, s^2 = 1 + dU/(E c^2):
 			// dlogT/ddU = (1-s)/(s(1+s)) * ds/ddU, ds/ddU = 1/(2 s E c^2)
@@ -382,7 +399,9 @@ template<class R> __device__ __forceinline__ int boundary_event(const DevTriangl
 	if ((ph & PH_ABSORB) && dU < 0.0f) {
 		// empirical absorption with probability exp(1 + E / (2 dU))
 		const float pa = expf(fa(1.0f, fdf(fm(0.5f, p.E), dU)));
-		if (rng.unit() < pa)
+		const float r = n_used ? u[1] : u[0];
+		++n_used;
+		if (r < pa)
 			return ST_TERMINATED;
 		if (score) {
 			// d log(1 - pa) / d dU = pa / (1 - pa) * E / (2 dU^2)

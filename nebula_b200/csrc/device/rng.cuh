@@ -64,11 +64,13 @@ __host__ __device__ __forceinline__ uint64_t child_lineage(uint64_t parent, uint
 	return z | 1ull;
 }
 
-// Uniform draws for one electron within one event.
+// Uniform draws for one electron within one event, four to a Philox block.
+// The events ask for whole blocks and take their draws by position, so that
+// the evaluation stands in the code a few times only, not at every draw, and
+// no draw indexes an array.
 struct PhiloxStream {
 	PhiloxKey key;
 	uint32_t c0base, tag, lin_lo, lin_hi;
-	uint32_t buf[4];
 	uint32_t n;   // draws taken in this event
 
 	__device__ __forceinline__ void init(PhiloxKey k, uint32_t event, uint32_t block0, uint32_t tag_,
@@ -81,15 +83,13 @@ struct PhiloxStream {
 		lin_hi = (uint32_t)(lineage >> 32);
 		n = 0;
 	}
-	__device__ __forceinline__ float unit()
+	// draws 4 b .. 4 b + 3
+	__device__ __forceinline__ void block(uint32_t b, float u[4]) const
 	{
-		const uint32_t j = n & 3u;
-		if (j == 0) {
-			buf[0] = c0base + (n >> 2); buf[1] = tag; buf[2] = lin_lo; buf[3] = lin_hi;
-			philox4x32_10(buf, key);
-		}
-		++n;
-		return u01_open(buf[j]);
+		uint32_t c[4] = { c0base + b, tag, lin_lo, lin_hi };
+		philox4x32_10(c, key);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) u[i] = u01_open(c[i]);
 	}
 };
 
@@ -98,11 +98,10 @@ struct PhiloxStream {
 struct ListStream {
 	const float* u;
 	uint32_t n, cap;
-	__device__ __forceinline__ float unit()
+	__device__ __forceinline__ void block(uint32_t b, float v[4]) const
 	{
-		const float v = n < cap ? u[n] : 0.5f;
-		++n;
-		return v;
+#pragma unroll
+		for (uint32_t i = 0; i < 4; ++i) v[i] = 4 * b + i < cap ? u[4 * b + i] : 0.5f;
 	}
 };
 

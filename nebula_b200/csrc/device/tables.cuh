@@ -19,28 +19,26 @@ __device__ __forceinline__ int clampi(int i, int lo, int hi) { return i < lo ? l
 // floorr (reference common/scalar_math.h:43-55): round toward -inf to int
 __device__ __forceinline__ int floor_to_int(float x) { return __float2int_rd(x); }
 
-__device__ __forceinline__ float tab(const DevTable& t, int i, int j, int k)
-{
-	return __ldg(t.data + ((size_t)i * t.ny + j) * t.nz + k);
-}
-
 __device__ __forceinline__ float table1_get(const DevTable& t, float x)
 {
 	const float xi = fm(fs(x, t.x_min), t.x_step);
 	const int lo = clampi(floor_to_int(xi), 0, t.nx - 2);
-	const float a = __ldg(t.data + lo), b = __ldg(t.data + lo + 1);
+	const float* const c = t.data + lo;
+	const float a = __ldg(c), b = __ldg(c + 1);
 	const float f = fs(xi, (float)lo);
 	return fa(fm(fs(1.0f, f), a), fm(f, b));
 }
 
+// (two-dimensional tables have nz = 1)
 __device__ __forceinline__ float table2_get(const DevTable& t, float x, float y)
 {
 	const float xi = fm(fs(x, t.x_min), t.x_step);
 	const float yi = fm(fs(y, t.y_min), t.y_step);
 	const int lx = clampi(floor_to_int(xi), 0, t.nx - 2);
 	const int ly = clampi(floor_to_int(yi), 0, t.ny - 2);
-	const float v00 = tab(t, lx, ly, 0), v10 = tab(t, lx + 1, ly, 0);
-	const float v01 = tab(t, lx, ly + 1, 0), v11 = tab(t, lx + 1, ly + 1, 0);
+	const float* const c = t.data + ((int64_t)lx * t.ny + ly);
+	const float* const c1 = c + t.ny;
+	const float v00 = __ldg(c), v10 = __ldg(c1), v01 = __ldg(c + 1), v11 = __ldg(c1 + 1);
 	const float fx = fs(xi, (float)lx), fy = fs(yi, (float)ly);
 	const float gx = fs(1.0f, fx), gy = fs(1.0f, fy);
 	// ((gx*gy)*v00 + (fx*gy)*v10) + (gx*fy)*v01) + (fx*fy)*v11
@@ -55,7 +53,8 @@ __device__ __forceinline__ float table2_rounddown(const DevTable& t, float x, fl
 {
 	const float xi = fm(fs(x, t.x_min), t.x_step);
 	const float yi = fm(fs(y, t.y_min), t.y_step);
-	return tab(t, clampi(floor_to_int(xi), 0, t.nx - 1), clampi(floor_to_int(yi), 0, t.ny - 1), 0);
+	return __ldg(t.data + ((int64_t)clampi(floor_to_int(xi), 0, t.nx - 1) * t.ny
+		+ clampi(floor_to_int(yi), 0, t.ny - 1)));
 }
 
 __device__ __forceinline__ float table3_get(const DevTable& t, float x, float y, float z)
@@ -66,10 +65,12 @@ __device__ __forceinline__ float table3_get(const DevTable& t, float x, float y,
 	const int lx = clampi(floor_to_int(xi), 0, t.nx - 2);
 	const int ly = clampi(floor_to_int(yi), 0, t.ny - 2);
 	const int lz = clampi(floor_to_int(zi), 0, t.nz - 2);
-	const float v000 = tab(t, lx, ly, lz), v100 = tab(t, lx + 1, ly, lz);
-	const float v010 = tab(t, lx, ly + 1, lz), v110 = tab(t, lx + 1, ly + 1, lz);
-	const float v001 = tab(t, lx, ly, lz + 1), v101 = tab(t, lx + 1, ly, lz + 1);
-	const float v011 = tab(t, lx, ly + 1, lz + 1), v111 = tab(t, lx + 1, ly + 1, lz + 1);
+	const float* const c = t.data + (((int64_t)lx * t.ny + ly) * t.nz + lz);
+	const float* const cx = c + (int64_t)t.ny * t.nz;
+	const float* const cy = c + t.nz;
+	const float* const cxy = cx + t.nz;
+	const float v000 = __ldg(c), v100 = __ldg(cx), v010 = __ldg(cy), v110 = __ldg(cxy);
+	const float v001 = __ldg(c + 1), v101 = __ldg(cx + 1), v011 = __ldg(cy + 1), v111 = __ldg(cxy + 1);
 	const float fx = fs(xi, (float)lx), fy = fs(yi, (float)ly), fz = fs(zi, (float)lz);
 	const float gx = fs(1.0f, fx), gy = fs(1.0f, fy), gz = fs(1.0f, fz);
 	// each term is ((a*b)*c)*v, summed left to right (table_3D.inl:100-109)
@@ -89,8 +90,8 @@ __device__ __forceinline__ float table3_rounddown(const DevTable& t, float x, fl
 	const float xi = fm(fs(x, t.x_min), t.x_step);
 	const float yi = fm(fs(y, t.y_min), t.y_step);
 	const float zi = fm(fs(z, t.z_min), t.z_step);
-	return tab(t, clampi(floor_to_int(xi), 0, t.nx - 1), clampi(floor_to_int(yi), 0, t.ny - 1),
-		clampi(floor_to_int(zi), 0, t.nz - 1));
+	return __ldg(t.data + (((int64_t)clampi(floor_to_int(xi), 0, t.nx - 1) * t.ny
+		+ clampi(floor_to_int(yi), 0, t.ny - 1)) * t.nz + clampi(floor_to_int(zi), 0, t.nz - 1)));
 }
 
 }  // namespace nbl

@@ -48,7 +48,7 @@ struct DevGeometry {
 
 // A table in the reference's transformed domain: row-major data, index per
 // axis = (v - v_min) * v_step (common/util/table_{1,2,3}D).
-struct DevTable {
+struct alignas(16) DevTable {
 	const float* data;
 	int32_t nx, ny, nz, pad;
 	float x_min, x_step, y_min, y_step, z_min, z_step;

@@ -237,13 +237,15 @@ __global__ void k_event_kat(const DevGeometry g, const DevMaterial* __restrict__
 	bool spawned = false;
 	Electron se;
 	se.pos = v3(0, 0, 0); se.dir = v3(0, 0, 0); se.E = 0;
+	float u[4];
+	rng.block(0, u);
 	if (kind == 3) {
 		const DevTriangle T = load_tri(g.tris, tri[i]);
-		st = boundary_event(T, mats, p, mat, rng, nullptr, ph);
-	} else if (kind == 1) {
-		spawned = inelastic_event(mats[mat], p, se, rng, ph);
+		st = boundary_event(T, mats, p, mat, u, rng.n, nullptr, ph);
+	} else if (kind == 1 && (ph & PH_KIEFT)) {
+		spawned = kieft_event(mats[mat], p, se, u, rng, ph);
 	} else {
-		elastic_event(mats[mat], p, rng, ph);
+		spawned = scatter_event(kind == 2, mats[mat], p, se, u, rng, ph);
 	}
 	float* o = state_out + 7 * i;
 	o[0] = p.pos.x; o[1] = p.pos.y; o[2] = p.pos.z; o[3] = p.dir.x; o[4] = p.dir.y; o[5] = p.dir.z; o[6] = p.E;
@@ -268,18 +270,28 @@ cudaError_t launch_event_kat(const DevGeometry& g, const DevMaterial* mats, uint
 }
 
 /* ----------------------------------------------------------- transport */
-// Event counters of one block, in shared memory (one shared atomic per
-// counted event), flushed to the device counters once per block and launch.
+// Event counters.  Those that every chunk counts are kept by the warp: lane k
+// adds counter k's lanes to its one register (a ballot and a population count
+// where the whole warp is converged), and adds the sum to the block's shared
+// counters when the warp has no more work.  Rare ones go there directly.  The
+// block's sums are flushed to the device counters once per launch.
 struct LocalCounters {
 	uint32_t* c;   // shared, N_COUNTERS words
-	// one shared atomic per group of lanes counting together
-	__device__ __forceinline__ void add(int k)
+	uint32_t acc;  // this lane's counter
+	__device__ __forceinline__ void count(int k, bool pred)
 	{
-		const cg::coalesced_group g = cg::coalesced_threads();
-		if (g.thread_rank() == 0)
-			atomicAdd(c + k, g.size());
+		const int n = __popc(__ballot_sync(0xffffffffu, pred));
+		if ((int)(threadIdx.x & 31u) == k)
+			acc += (uint32_t)n;
+	}
+	__device__ __forceinline__ void rare(int k) { atomicAdd(c + k, 1u); }
+	__device__ __forceinline__ void flush()
+	{
+		if ((threadIdx.x & 31u) < N_COUNTERS && acc)
+			atomicAdd(c + (threadIdx.x & 31u), acc);
 	}
 };
+static_assert(N_COUNTERS <= 32, "one lane per counter");
 
 // What one electron needs to know about the run it belongs to: its geometry
 // and its random-number key (a batched run holds one of each per job).
@@ -317,16 +329,15 @@ __device__ __forceinline__ void store_resume(const Queue& q, uint32_t i, const F
 }
 
 // The checks a flight starts with: NaN state, domain, event budget, energy cut
-// (in that order; the flight is counted first).  False: the electron ends here.
+// (in that order).  False: the electron ends here.
 template<bool ADJ>
 __device__ __forceinline__ bool flight_begin(const StepParams& P, const DevGeometry& G, const Electron& p, int mat,
 	uint32_t& event, LocalCounters& lc, const float* dbar, const DevMaterial* mats)
 {
-	lc.add(CNT_FLIGHTS);
-	if (!(p.E == p.E) || !(p.pos.x == p.pos.x)) { lc.add(CNT_NAN); return false; }
+	if (!(p.E == p.E) || !(p.pos.x == p.pos.x)) { lc.rare(CNT_NAN); return false; }
 	if (!in_domain(G, p.pos.x, p.pos.y, p.pos.z))
 		return false;
-	if (event >= P.max_events) { lc.add(CNT_EVENT_BUDGET); return false; }
+	if (event >= P.max_events) { lc.rare(CNT_EVENT_BUDGET); return false; }
 	++event;
 	if (mat >= 0) {
 		const float barrier = (ADJ && dbar && mat < 2) ? fa(mats[mat].barrier, dbar[mat]) : mats[mat].barrier;
@@ -336,95 +347,80 @@ __device__ __forceinline__ bool flight_begin(const StepParams& P, const DevGeome
 	return true;
 }
 
-// Free flight(s) of an electron whose flight_begin passed: free-path sampling,
-// octree walk, move.  Flights in vacuum that hit nothing end without an event
-// and are repeated (the next one leaves the domain).
-// Returns the queue of the event the flight ends in, -1 when the electron is
-// terminated, or EV_WALK when the walk reached the run's per-iteration cell
-// budget (`fr` then holds where it stands).  With `resume` non-null, the
-// flight stored at entry `resume_i` of that walk queue continues (its checks,
-// event count and random draws are behind it).
+// Free flight of an electron whose flight_begin passed: free-path sampling,
+// octree walk, move.  Returns the queue of the event the flight ends in, -1
+// when the electron is terminated, or EV_WALK when the walk reached the run's
+// per-iteration cell budget (`fr` then holds where it stands).  With `resume`,
+// the flight stored in `fr` continues (its checks, event count and random
+// draws are behind it).  A flight in vacuum that hits nothing ends without an
+// event and is repeated (`repeats`; the next one leaves the domain as a rule,
+// else it is queued as a walk that has not started, four flights in all).
 // Mirrors cpu_driver::init / kernels::init
 // (drivers/cpu/cpu_driver.inl:74-130, drivers/gpu/gpu_driver.inl:403-480).
 template<bool ADJ>
 __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& rv, Electron& p, int mat, int& last_tri,
 	uint32_t& event, uint32_t stream_tag, uint64_t lineage, float* sc, LocalCounters& lc, const float* dbar,
-	FlightResume& fr, const Queue* resume, uint32_t resume_i, const DevMaterial* mats)
+	FlightResume& fr, bool resume, const DevMaterial* mats, int& repeats)
 {
 	const DevGeometry& G = *rv.geom;
-	if (resume) {
-		load_resume(*resume, resume_i, fr);
-		lc.add(CNT_RESUMED);
+	const DevMaterial* const m = mats + mat;              // read for mat >= 0 only
+	float mu_el = 0.0f, mu_in = 0.0f;
+	if (!resume) {
+		fr.hop = 0;
+		fr.type = 0;
+		fr.dist = G.max_extent;
+		if (mat >= 0) {
+			PhiloxStream r;
+			r.init(rv.key, event, 0u, stream_tag, lineage);
+			float u[4];
+			r.block(0, u);
+			const float pe = sample_path(m->el_imfp, m->el_scale, p.E, u[0], mu_el);
+			const float pi = sample_path(m->in_imfp, m->in_scale, p.E, u[1], mu_in);
+			fr.dist = __int_as_float(0x7f800000);
+			if (pe < fr.dist) { fr.dist = pe; fr.type = 2; }
+			if (pi < fr.dist) { fr.dist = pi; fr.type = 1; }
+		}
+		fr.w = walk_start(p.pos.x, p.pos.y, p.pos.z, fr.dist);
 	}
-	bool begun = true;
-	for (int hop = resume ? fr.hop : 0; hop < 4; ++hop) {
-		int type = 0;
-		float dist;
-		float mu_el = 0.0f, mu_in = 0.0f;
-		const DevMaterial* m = nullptr;
-		WalkState w;
+	const V3 d = vnormalised(p.dir);
+	float idist;
+	const int hit = propagate_cells(G, fr.w, d.x, d.y, d.z, fr.dist, last_tri, mat, idist, (int)P.walk_cells);
+	if (hit == NBL_WALK_PENDING)
+		return EV_WALK;
+	if (hit == -2) { lc.rare(CNT_WALK_OVERFLOW); return -1; }
+	if (ADJ && mat >= 0 && mat < 2) {
+		// score of the flight: density mu_k exp(-(mu_in+mu_el) d) of the
+		// chosen event k at distance d, or survival exp(-(mu_in+mu_el) d)
+		// when a boundary cuts the flight; derivative w.r.t. the scales
 		if (resume) {
-			resume = nullptr;
-			begun = false;
-			type = fr.type;
-			dist = fr.dist;
-			w = fr.w;
-			if (mat >= 0) {
-				m = mats + mat;
-				if (ADJ) {
-					// the inverse mean free paths the flight was sampled with
-					mu_el = imfp_at(m->el_imfp, m->el_scale, p.E);
-					mu_in = imfp_at(m->in_imfp, m->in_scale, p.E);
-				}
-			}
-		} else {
-			if (!begun && !flight_begin<ADJ>(P, G, p, mat, event, lc, dbar, mats))
-				return -1;
-			begun = false;
-			dist = G.max_extent;
-			if (mat >= 0) {
-				m = mats + mat;
-				PhiloxStream r;
-				r.init(rv.key, event, 0u, stream_tag, lineage);
-				const float pe = sample_path(m->el_imfp, m->el_scale, p.E, r, mu_el);
-				const float pi = sample_path(m->in_imfp, m->in_scale, p.E, r, mu_in);
-				dist = __int_as_float(0x7f800000);
-				if (pe < dist) { dist = pe; type = 2; }
-				if (pi < dist) { dist = pi; type = 1; }
-			}
-			w = walk_start(p.pos.x, p.pos.y, p.pos.z, dist);
+			// the inverse mean free paths the flight was sampled with
+			mu_el = imfp_at(m->el_imfp, m->el_scale, p.E);
+			mu_in = imfp_at(m->in_imfp, m->in_scale, p.E);
 		}
-		const V3 d = vnormalised(p.dir);
-		float idist;
-		const int hit = propagate_cells(G, w, d.x, d.y, d.z, dist, last_tri, mat, idist, (int)P.walk_cells);
-		if (hit == NBL_WALK_PENDING) {
-			fr.w = w;
-			fr.dist = dist;
-			fr.type = type;
-			fr.hop = hop;
-			return EV_WALK;
-		}
-		if (hit == -2) { lc.add(CNT_WALK_OVERFLOW); return -1; }
-		if (ADJ && mat >= 0 && mat < 2) {
-			// score of the flight: density mu_k exp(-(mu_in+mu_el) d) of the
-			// chosen event k at distance d, or survival exp(-(mu_in+mu_el) d)
-			// when a boundary cuts the flight; derivative w.r.t. the scales
-			const float travel = hit >= 0 ? idist : dist;
-			const float in_k = (hit < 0 && type == 1) ? 1.0f : 0.0f;
-			const float el_k = (hit < 0 && type == 2) ? 1.0f : 0.0f;
-			sc[3 * mat + 0] += (in_k - mu_in * travel) / m->in_scale;
-			sc[3 * mat + 1] += (el_k - mu_el * travel) / m->el_scale;
-		}
-		if (hit >= 0) {
-			p.pos = vadd(p.pos, vmul(d, idist));
-			last_tri = hit;
-			return EV_BOUNDARY;
-		}
-		p.pos = vadd(p.pos, vmul(d, dist));
-		if (type == 1) return EV_INELASTIC;
-		if (type == 2) return EV_ELASTIC;
+		const float travel = hit >= 0 ? idist : fr.dist;
+		const float in_k = (hit < 0 && fr.type == 1) ? 1.0f : 0.0f;
+		const float el_k = (hit < 0 && fr.type == 2) ? 1.0f : 0.0f;
+		const float s_in = (in_k - mu_in * travel) / m->in_scale, s_el = (el_k - mu_el * travel) / m->el_scale;
+		if (mat == 0) { sc[0] += s_in; sc[1] += s_el; }
+		else { sc[3] += s_in; sc[4] += s_el; }
 	}
-	return -1;
+	if (hit >= 0) {
+		p.pos = vadd(p.pos, vmul(d, idist));
+		last_tri = hit;
+		return EV_BOUNDARY;
+	}
+	p.pos = vadd(p.pos, vmul(d, fr.dist));
+	if (fr.type == 1) return EV_INELASTIC;
+	if (fr.type == 2) return EV_ELASTIC;
+	if (fr.hop == 3)
+		return -1;
+	++repeats;
+	if (!flight_begin<ADJ>(P, G, p, mat, event, lc, dbar, mats))
+		return -1;
+	++fr.hop;
+	fr.dist = G.max_extent;
+	fr.w = walk_start(p.pos.x, p.pos.y, p.pos.z, fr.dist);
+	return EV_WALK;
 }
 
 __device__ __forceinline__ void store_electron(const Queue& q, uint32_t slot, const Electron& p, int mat, int last_tri,
@@ -467,9 +463,8 @@ __device__ __noinline__ void detection_output(const StepParams* Pp, const BatchP
 	uint32_t rec_index, uint32_t job, PhiloxKey key, uint32_t stream_tag, Scores sc, bool wshift, uint32_t* s_counters)
 {
 	const StepParams& P = *Pp;
-	LocalCounters lc{ s_counters };
+	LocalCounters lc{ s_counters, 0u };
 	if (det) {
-		lc.add(CNT_DETECTED);
 		const Tallies& T = P.tal;
 		if (BATCH) {
 			atomicAdd((p.E < 50.0f ? Bp->job_se : Bp->job_bse) + job, 1ull);
@@ -518,7 +513,7 @@ __device__ __noinline__ void detection_output(const StepParams* Pp, const BatchP
 				if (BATCH && P.det_job)
 					P.det_job[rslot] = (uint8_t)job;
 			} else {
-				lc.add(CNT_RECORD_OVERFLOW);
+				lc.rare(CNT_RECORD_OVERFLOW);
 			}
 		}
 	}
@@ -549,7 +544,7 @@ __device__ __forceinline__ void deposit(const StepParams& P, bool scat, const El
 				r.px = pr->px; r.py = pr->py;
 				P.dep[slot] = r;
 			} else {
-				lc.add(CNT_DEPOSIT_OVERFLOW);
+				lc.rare(CNT_DEPOSIT_OVERFLOW);
 			}
 		}
 	}
@@ -573,8 +568,7 @@ __device__ __forceinline__ void deposit(const StepParams& P, bool scat, const El
 		}
 		__syncwarp();
 	}
-	if (scat)
-		lc.add(CNT_DEPOSITS);
+	lc.count(CNT_DEPOSITS, scat);
 }
 
 template<bool ADJ, bool BATCH, bool DEP = false, uint32_t PHC = 0u>
@@ -698,7 +692,6 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 			} else {
 				tag = P.tag_base + qi;
 			}
-			lc.add(CNT_PRIMARIES);
 		}
 		const float e_before = p.E;
 		// run context: job geometry / key, the primary's record, the tag that
@@ -733,36 +726,40 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 		int status = (kind >= 0) ? ST_RUNNING : ST_TERMINATED;
 		bool spawn = false;
 		Electron se;
-		if (kind == EV_BOUNDARY) {
-			lc.add(CNT_BOUNDARY);
+		if (kind >= EV_BOUNDARY && kind <= EV_INELASTIC) {
 			PhiloxStream r;
 			r.init(rv.key, event, 1u, stream_tag, lineage);
-			const DevTriangle T = load_tri(rv.geom->tris, last_tri);
-			if (ADJ) {
-				BoundaryScore bs = { 0.0f, 0.0f, -1, -1 };
-				status = boundary_event(T, mats, p, mat, r, &bs, phys, wshift ? dbar : nullptr);
-				// the work function enters through barrier = fermi + W of the
-				// materials on either side of the crossing
-				if (!wshift) {
-					if (bs.mat_in >= 0 && bs.mat_in < 2) sc[3 * bs.mat_in + 2] += bs.d_in;
-					if (bs.mat_out >= 0 && bs.mat_out < 2) sc[3 * bs.mat_out + 2] += bs.d_out;
+			float u[4];
+			r.block(0, u);
+			if (kind == EV_BOUNDARY) {
+				const DevTriangle T = load_tri(rv.geom->tris, last_tri);
+				if (ADJ) {
+					BoundaryScore bs = { 0.0f, 0.0f, -1, -1 };
+					status = boundary_event(T, mats, p, mat, u, r.n, &bs, phys, wshift ? dbar : nullptr);
+					// the work function enters through barrier = fermi + W of the
+					// materials on either side of the crossing
+					if (!wshift) {
+						if (bs.mat_in == 0) sc[2] += bs.d_in;
+						if (bs.mat_in == 1) sc[5] += bs.d_in;
+						if (bs.mat_out == 0) sc[2] += bs.d_out;
+						if (bs.mat_out == 1) sc[5] += bs.d_out;
+					}
+				} else {
+					status = boundary_event(T, mats, p, mat, u, r.n, nullptr, phys);
 				}
 			} else {
-				status = boundary_event(T, mats, p, mat, r, nullptr, phys);
+				last_tri = -1;
+				if (kind == EV_INELASTIC && (phys & PH_KIEFT))
+					spawn = kieft_event(mats[mat], p, se, u, r, phys);
+				else
+					spawn = scatter_event(kind == EV_ELASTIC, mats[mat], p, se, u, r, phys);
 			}
-		} else if (kind == EV_ELASTIC) {
-			lc.add(CNT_ELASTIC);
-			last_tri = -1;
-			PhiloxStream r;
-			r.init(rv.key, event, 1u, stream_tag, lineage);
-			elastic_event(mats[mat], p, r, phys);
-		} else if (kind == EV_INELASTIC) {
-			lc.add(CNT_INELASTIC);
-			last_tri = -1;
-			PhiloxStream r;
-			r.init(rv.key, event, 1u, stream_tag, lineage);
-			spawn = inelastic_event(mats[mat], p, se, r, phys);
 		}
+		lc.count(CNT_PRIMARIES, kind == K_PRIMARY);
+		lc.count(CNT_RESUMED, kind == EV_WALK);
+		lc.count(CNT_BOUNDARY, kind == EV_BOUNDARY);
+		lc.count(CNT_ELASTIC, kind == EV_ELASTIC);
+		lc.count(CNT_INELASTIC, kind == EV_INELASTIC);
 
 		// energy deposit of a scatter event that changed the energy
 		if (DEP)
@@ -772,6 +769,7 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 		// detection output: record + tallies (out of line: a warp has a
 		// detection in a small fraction of its chunks)
 		if (__any_sync(0xFFFFFFFFu, status == ST_DETECTED)) {
+			lc.count(CNT_DETECTED, status == ST_DETECTED);
 			Scores scs;
 #pragma unroll
 			for (int k = 0; k < 6; ++k) scs.v[k] = ADJ ? sc[k] : 0.0f;
@@ -782,8 +780,9 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 		// secondary: inherits material, tag and the parent's scores; its
 		// lineage id is derived from the parent's and the spawning event
 		uint64_t se_lineage = 0;
+		lc.count(CNT_SPAWNED, spawn);
+		bool cut = false;
 		if (spawn) {
-			lc.add(CNT_SPAWNED);
 			se_lineage = child_lineage(lineage, event);
 			// A secondary below its material's escape threshold ends at its
 			// first free flight (energy cut, before any random draw or
@@ -793,18 +792,19 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 			const float barrier = (wshift && mat < 2) ? fa(mats[mat].barrier, dbar[mat]) : mats[mat].barrier;
 			if (se.E < fa(barrier, P.energy_threshold)) {
 				spawn = false;
-				lc.add(CNT_FLIGHTS);
-				lc.add(CNT_TERMINATED);
+				cut = true;
 			}
 		}
+		lc.count(CNT_FLIGHTS, cut);
+		lc.count(CNT_TERMINATED, cut);
 
 		// The checks the electron's own next flight starts with (a continued
 		// walk is past them).
 		bool flying = status == ST_RUNNING;
 		if (flying && kind != EV_WALK)
 			flying = flight_begin<ADJ>(P, *rv.geom, p, mat, event, lc, wshift ? dbar : nullptr, mats);
-		if (kind >= 0 && status != ST_DETECTED && !flying)
-			lc.add(CNT_TERMINATED);
+		lc.count(CNT_FLIGHTS, status == ST_RUNNING && kind != EV_WALK);
+		lc.count(CNT_TERMINATED, kind >= 0 && status != ST_DETECTED && !flying);
 
 		// Half of the electrons end at the energy cut right after an inelastic
 		// event, and half of the events leave a secondary: a lane whose electron
@@ -870,9 +870,9 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 					dbar[1] = fm(P.wstep, wsign(rv.key, stream_tag, 1));
 				}
 				flying = flight_begin<ADJ>(P, *rv.geom, p, mat, event, lc, wshift ? dbar : nullptr, mats);
-				if (!flying)
-					lc.add(CNT_TERMINATED);
 			}
+			lc.count(CNT_FLIGHTS, take);
+			lc.count(CNT_TERMINATED, take && !flying);
 		}
 		// The flight queue's counter hands out the tickets: the first
 		// se_budget secondaries are queued, later ones go to the spill ring
@@ -887,13 +887,13 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 			uint32_t at = 0;
 			if (queued) {
 				if (sslot < P.qcap) { dst = &qout[EV_NEW]; at = sslot; }
-				else lc.add(CNT_QUEUE_OVERFLOW);
+				else lc.rare(CNT_QUEUE_OVERFLOW);
 			} else {
-				lc.add(CNT_SPILLED);
+				lc.rare(CNT_SPILLED);
 				// the ring holds at most spill_mask + 1 electrons, counting the
 				// ones being drained during this iteration
 				if (sp_tail + pslot - sp_head <= P.spill_mask) { dst = &P.spill; at = (sp_tail + pslot) & P.spill_mask; }
-				else lc.add(CNT_QUEUE_OVERFLOW);
+				else lc.rare(CNT_QUEUE_OVERFLOW);
 			}
 			if (dst) {
 				store_electron(*dst, at, se, mat, -1, tag, 0u, se_lineage);
@@ -905,12 +905,24 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 		}
 
 		// next free flight (or the rest of a walk cut short last iteration)
-		int qtype = -1;
+		int qtype = -1, repeats = 0;
+		if (kind == EV_WALK)
+			load_resume(qin[EV_WALK], qi, fr);
 		if (flying)
 			qtype = free_flight<ADJ>(P, rv, p, mat, last_tri, event, stream_tag, lineage, sc, lc,
-				wshift ? dbar : nullptr, fr, kind == EV_WALK ? &qin[EV_WALK] : nullptr, qi, mats);
-		if (flying && qtype < 0)
-			lc.add(CNT_TERMINATED);
+				wshift ? dbar : nullptr, fr, kind == EV_WALK, mats, repeats);
+		const unsigned ended = __ballot_sync(0xFFFFFFFFu, flying && qtype < 0);
+		if (ended) {
+			if (lane == (uint32_t)CNT_TERMINATED)
+				lc.acc += (uint32_t)__popc(ended);
+			// (an electron that repeats a flight ends in it as a rule)
+			const uint32_t again = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)repeats);
+			if (lane == (uint32_t)CNT_FLIGHTS)
+				lc.acc += again;
+			repeats = 0;
+		}
+		if (repeats)
+			atomicAdd(lc.c + CNT_FLIGHTS, (uint32_t)repeats);
 		{
 			// the warp's next chunk is claimed (lane 5) together with the
 			// queue slots (lanes 0-4): one atomic round trip for both
@@ -919,7 +931,7 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 				next = atomicAdd(work, 32u);
 			const uint32_t slot = warp_reserve5(cw, qtype);
 			if (qtype >= 0 && slot >= P.qcap)
-				lc.add(CNT_QUEUE_OVERFLOW);
+				lc.rare(CNT_QUEUE_OVERFLOW);
 			// compile-time queue indices (a run-time index into the kernel
 			// parameters would copy them to local memory)
 #pragma unroll
@@ -970,8 +982,9 @@ static void allow_shared_bytes(const void* kernel, size_t bytes)
 		cudaGetLastError();
 }
 
-__device__ __forceinline__ void flush_counters(const StepParams& P, uint32_t* s_counters)
+__device__ __forceinline__ void flush_counters(const StepParams& P, LocalCounters& lc, uint32_t* s_counters)
 {
+	lc.flush();
 	__syncthreads();
 	for (int k = threadIdx.x; k < N_COUNTERS; k += blockDim.x)
 		if (s_counters[k])
@@ -993,13 +1006,13 @@ __global__ void __launch_bounds__(256, NBL_STEP_MIN_BLOCKS) k_step(const __grid_
 	for (int k = threadIdx.x; k < N_COUNTERS; k += blockDim.x)
 		s_counters[k] = 0u;
 	__syncthreads();
-	LocalCounters lc{ s_counters };
+	LocalCounters lc{ s_counters, 0u };
 	const BatchParams none{};
 	// materials read from global memory: staged in shared memory as the
 	// batched kernel stages them, this kernel measured slower (-0.4 % on the
 	// grating scan, -1.5 % on the 1.2 M-triangle mesh)
 	step_iteration<ADJ, false, DEP, PHC>(P, none, it, lc, P.mats, s_rank + (threadIdx.x & ~31u), s_lane);
-	flush_counters(P, s_counters);
+	flush_counters(P, lc, s_counters);
 }
 
 // Grid-wide barrier of the persistent kernel (all blocks co-resident by the
@@ -1058,7 +1071,7 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 		s_jobs[k] = B.jobs[k];
 	const DevMaterial* s_mats = stage_materials(P);
 	__syncthreads();
-	LocalCounters lc{ s_counters };
+	LocalCounters lc{ s_counters, 0u };
 	uint32_t it = 0;
 	for (; it < B.max_iterations; ++it) {
 		if (!step_iteration<ADJ, true, false, PHC>(P, B, it, lc, s_mats, s_rank + (threadIdx.x & ~31u), nullptr, s_geoms, s_jobs))
@@ -1071,7 +1084,7 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 		if (it >= B.max_iterations)
 			atomicOr(B.err, 2u);
 	}
-	flush_counters(P, s_counters);
+	flush_counters(P, lc, s_counters);
 }
 
 // The step kernel instantiation a run's parameters select: adjoint or not,
