@@ -250,7 +250,8 @@ typedef struct nbl_params {
 	nbl_image_filter image_filter; /* detector acceptance of the per-pixel images */
 	uint32_t walk_cells;         /* leaf cells a flight's octree walk takes per iteration; a longer walk
 	                                continues in the next iteration from where it stopped (same cells,
-	                                same float values, same results); 0: 1 */
+	                                same float values, same results); on fine meshes empty cells may
+	                                come along with each; 0: 1 */
 } nbl_params;
 void nbl_params_defaults(nbl_params* p);
 

@@ -353,7 +353,9 @@ __device__ __forceinline__ int boundary_event(const DevTriangle& T, const DevMat
 	const float* dbar = nullptr)
 {
 	const V3 nd = vnormalised(p.dir);
-	const V3 n = vnormalised(v3(T.nx, T.ny, T.nz));
+	V3 n;
+	tri_normal(T, n.x, n.y, n.z);
+	n = vnormalised(n);
 	const float c = vdot(n, nd);
 	int min_, mout;
 	if (c > 0.0f) { min_ = T.mat_in; mout = T.mat_out; } else { min_ = T.mat_out; mout = T.mat_in; }

@@ -861,6 +861,7 @@ nbl_status nbl_sim_create(const nbl_geometry* g, nbl_material* const* materials,
 		const bool adj = params->adjoint != 0;
 		require(params->walk_cells <= (1u << 20), "walk_cells must be at most 2^20");
 		sp.walk_cells = params->walk_cells ? params->walk_cells : 1u;
+		sp.pass_empty = fine_mesh(g->g) ? PASS_EMPTY : 0;
 		for (int b = 0; b < 2; ++b)
 			for (int q = 0; q < N_QUEUES; ++q) {
 				DevBuf* qb = s->queues[b][q];

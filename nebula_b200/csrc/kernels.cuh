@@ -58,6 +58,15 @@ struct Tallies {
 	float cos_min, cos_max;
 };
 
+// Empty leaves a walk passes before each cell of its budget, on a fine mesh.
+// On the 1.2 M-triangle rough lines a flight crosses 2.6 leaves and 80 % of
+// them are empty: a lane with an empty one waits while its warp's others test
+// lists of 10 to 16 triangles, and is then queued again for one cell.
+// On the 4 k-triangle grating a leaf near the surface is hardly ever empty.
+// Rough lines, 128 x 128 x 100: 70.7 ms without, 64.9 with one, 64.5 with two,
+// 66.0 with three; grating 160 x 160 x 100: 68.5 ms without, 71.8 with one.
+constexpr int PASS_EMPTY = 2;
+
 struct StepParams {
 	DevGeometry geom;
 	const DevMaterial* mats;
@@ -95,6 +104,7 @@ struct StepParams {
 	float g_org[3], g_inv[3]; // grid origin, 1 / voxel size
 	int32_t gn[3];
 	uint32_t walk_cells;      // leaf cells a flight's walk takes per iteration before it continues in the next
+	int32_t pass_empty;       // empty leaves passed before each of them (0 or PASS_EMPTY)
 };
 
 // Work-function sign of a primary for material m (0 or 1): +1 or -1 from a

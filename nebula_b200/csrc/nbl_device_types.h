@@ -22,23 +22,29 @@ struct PhiloxKey { uint32_t k0, k1; };
 // stopped at the per-iteration cell budget and continues.
 enum : int32_t { EV_BOUNDARY = 0, EV_ELASTIC = 1, EV_INELASTIC = 2, EV_NEW = 3, EV_WALK = 4, N_QUEUES = 5 };
 
-// One triangle, 64 bytes, four 16-byte vectors so a warp fetches it with
-// 128-bit loads: (r0, material_in) (e1, material_out) (e2, 0) (normal, 0).
-// r0/e1/e2 are the reference triangle's members (core/triangle.h:70-76);
-// normal = cross(e1, e2) computed once in float on the host with the same
-// operations as triangle::get_normal (core/triangle.inl:75-78), so it is the
-// value the reference recomputes per test.
+// One triangle, 48 bytes, three 16-byte vectors: (r0, material_in)
+// (e1, material_out) (e2, 0).  r0/e1/e2 are the reference triangle's members
+// (core/triangle.h:70-76).
 struct DevTriangle {
 	float r0x, r0y, r0z; int32_t mat_in;
 	float e1x, e1y, e1z; int32_t mat_out;
 	float e2x, e2y, e2z; int32_t pad0;
-	float nx, ny, nz; int32_t pad1;
 };
-static_assert(sizeof(DevTriangle) == 64, "DevTriangle must be 64 bytes");
+static_assert(sizeof(DevTriangle) == 48, "DevTriangle must be 48 bytes");
+
+// A triangle's plane, 16 bytes, in an array of its own: the walk's first pass
+// over a leaf's list reads only this (8 planes per cache line).  (x, y, z) is
+// the unit normal and w its product with r0, all divided by the distance the
+// ray test's float rounding can shift the triangle's plane by (plane_of in
+// host/device.hpp), so that a ray farther than 1 from the plane is past any
+// rounding.  NaN for a triangle without a normal: no comparison rejects it.
+struct DevPlane { float x, y, z, w; };
+static_assert(sizeof(DevPlane) == 16, "DevPlane must be 16 bytes");
 
 struct DevGeometry {
 	const int32_t* octree;       // reference linearized layout (octree_builder.h:222-231)
 	const DevTriangle* tris;
+	const DevPlane* planes;      // [n_tri]
 	float cx, cy, cz;            // root AABB centre
 	float hx, hy, hz;            // root AABB half size
 	float max_extent;            // 2 |halfsize| as the reference computes it

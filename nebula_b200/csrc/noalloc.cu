@@ -36,7 +36,7 @@
 #include <algorithm>
 
 #include "kernels.cuh"
-#include "host/internal.hpp"
+#include "host/device.hpp"
 
 namespace nbl {
 namespace {
@@ -142,7 +142,7 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 		require(max_mat < n_materials, "geometry uses more materials than given");
 		const HostGeometry& hg = g->g;
 		const size_t oct_bytes = align_up(hg.octree.size() * sizeof(int32_t));
-		require(oct_bytes + hg.tris.size() * sizeof(DevTriangle) <= NA_GEOM_BYTES,
+		require(oct_bytes + hg.tris.size() * (sizeof(DevTriangle) + sizeof(DevPlane)) <= NA_GEOM_BYTES,
 			"nbl_run_noalloc: geometry exceeds its " + std::to_string(NA_GEOM_BYTES >> 20) + " MiB budget");
 		size_t table_bytes = 0;
 		for (int i = 0; i < n_materials; ++i) {
@@ -168,26 +168,23 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 		unsigned char* base = scratch_address(params->device);
 		cudaStream_t s = static_cast<cudaStream_t>(params->stream);
 
-		// device copies of the geometry (64-byte triangles with normals) and tables
+		// device copies of the geometry (triangles, their planes) and tables
 		unsigned char* geom = base + OFF_GEOM;
 		cuda_ok(cudaMemcpyAsync(geom, hg.octree.data(), hg.octree.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s),
 			"copy octree");
+		unsigned char* planes = geom + oct_bytes + hg.tris.size() * sizeof(DevTriangle);
 		DevTriangle chunk[256];
+		DevPlane plane_chunk[256];
 		for (size_t i = 0; i < hg.tris.size(); i += 256) {
 			const size_t k = std::min<size_t>(256, hg.tris.size() - i);
 			for (size_t j = 0; j < k; ++j) {
-				const nbl_triangle& t = hg.tris[i + j];
-				DevTriangle& d = chunk[j];
-				d.r0x = t.r0[0]; d.r0y = t.r0[1]; d.r0z = t.r0[2]; d.mat_in = t.material_in;
-				d.e1x = t.e1[0]; d.e1y = t.e1[1]; d.e1z = t.e1[2]; d.mat_out = t.material_out;
-				d.e2x = t.e2[0]; d.e2y = t.e2[1]; d.e2z = t.e2[2]; d.pad0 = 0;
-				d.nx = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
-				d.ny = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
-				d.nz = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
-				d.pad1 = 0;
+				chunk[j] = device_triangle(hg.tris[i + j]);
+				plane_chunk[j] = plane_of(hg.tris[i + j], hg);
 			}
 			cuda_ok(cudaMemcpyAsync(geom + oct_bytes + i * sizeof(DevTriangle), chunk, k * sizeof(DevTriangle),
 				cudaMemcpyHostToDevice, s), "copy triangles");
+			cuda_ok(cudaMemcpyAsync(planes + i * sizeof(DevPlane), plane_chunk, k * sizeof(DevPlane),
+				cudaMemcpyHostToDevice, s), "copy planes");
 			cuda_ok(cudaStreamSynchronize(s), "copy triangles");
 		}
 		DevMaterial dm[NBL_NOALLOC_MAX_MATERIALS];
@@ -230,6 +227,7 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 		StepParams sp{};
 		sp.geom.octree = reinterpret_cast<const int32_t*>(geom);
 		sp.geom.tris = reinterpret_cast<const DevTriangle*>(geom + oct_bytes);
+		sp.geom.planes = reinterpret_cast<const DevPlane*>(planes);
 		sp.geom.cx = hg.center[0]; sp.geom.cy = hg.center[1]; sp.geom.cz = hg.center[2];
 		sp.geom.hx = hg.halfsize[0]; sp.geom.hy = hg.halfsize[1]; sp.geom.hz = hg.halfsize[2];
 		sp.geom.max_extent = hg.max_extent;

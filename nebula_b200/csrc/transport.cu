@@ -39,10 +39,6 @@
 #include <algorithm>
 namespace cg = cooperative_groups;
 
-#ifndef NBL_STEP_MIN_BLOCKS
-#define NBL_STEP_MIN_BLOCKS 4
-#endif
-
 namespace nbl {
 
 __device__ __forceinline__ unsigned lanemask_lt()
@@ -360,7 +356,7 @@ __device__ __forceinline__ bool flight_begin(const StepParams& P, const DevGeome
 template<bool ADJ>
 __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& rv, Electron& p, int mat, int& last_tri,
 	uint32_t& event, uint32_t stream_tag, uint64_t lineage, float* sc, LocalCounters& lc, const float* dbar,
-	FlightResume& fr, bool resume, const DevMaterial* mats, int& repeats)
+	FlightResume& fr, bool resume, const DevMaterial* mats, int pass_empty, int& repeats)
 {
 	const DevGeometry& G = *rv.geom;
 	const DevMaterial* const m = mats + mat;              // read for mat >= 0 only
@@ -384,7 +380,8 @@ __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& r
 	}
 	const V3 d = vnormalised(p.dir);
 	float idist;
-	const int hit = propagate_cells(G, fr.w, d.x, d.y, d.z, fr.dist, last_tri, mat, idist, (int)P.walk_cells);
+	const int hit = propagate_cells(G, fr.w, d.x, d.y, d.z, fr.dist, last_tri, mat, idist, (int)P.walk_cells,
+		pass_empty);
 	if (hit == NBL_WALK_PENDING)
 		return EV_WALK;
 	if (hit == -2) { lc.rare(CNT_WALK_OVERFLOW); return -1; }
@@ -571,7 +568,7 @@ __device__ __forceinline__ void deposit(const StepParams& P, bool scat, const El
 	lc.count(CNT_DEPOSITS, scat);
 }
 
-template<bool ADJ, bool BATCH, bool DEP = false, uint32_t PHC = 0u>
+template<bool ADJ, bool BATCH, bool DEP = false, uint32_t PHC = 0u, int FINE = 0>
 __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchParams& B, uint32_t it, LocalCounters& lc,
 	const DevMaterial* mats, uint8_t* s_rank, float* s_lane = nullptr, const DevGeometry* s_geoms = nullptr,
 	const DevJob* s_jobs = nullptr)
@@ -580,6 +577,8 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 	// for the default selection (its option tests fold away, and the code of
 	// the unselected inelastic model drops out), the run-time word otherwise
 	const uint32_t phys = PHC ? PHC : P.phys;
+	// likewise the empty leaves passed
+	const int pass_empty = FINE >= 0 ? FINE * PASS_EMPTY : P.pass_empty;
 	const uint32_t rs = it % 3u, ws = (it + 1u) % 3u, zs = (it + 2u) % 3u;
 	const uint32_t* cr = P.ctrl + rs * SLOT_WORDS;
 	uint32_t* cw = P.ctrl + ws * SLOT_WORDS;
@@ -910,7 +909,7 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 			load_resume(qin[EV_WALK], qi, fr);
 		if (flying)
 			qtype = free_flight<ADJ>(P, rv, p, mat, last_tri, event, stream_tag, lineage, sc, lc,
-				wshift ? dbar : nullptr, fr, kind == EV_WALK, mats, repeats);
+				wshift ? dbar : nullptr, fr, kind == EV_WALK, mats, pass_empty, repeats);
 		const unsigned ended = __ballot_sync(0xFFFFFFFFu, flying && qtype < 0);
 		if (ended) {
 			if (lane == (uint32_t)CNT_TERMINATED)
@@ -991,14 +990,16 @@ __device__ __forceinline__ void flush_counters(const StepParams& P, LocalCounter
 			atomicAdd(P.counters + k, (unsigned long long)s_counters[k]);
 }
 
-// One wavefront iteration per launch (the plain method).  Four resident
-// blocks of 256 threads per SM (at most 64 registers): the kernel is latency
-// bound, so warps in flight matter more than registers.
+// One wavefront iteration per launch (the plain method).
 // DEP: energy deposits on (a separate instantiation, so the plain step keeps
 // none of their code).  PHC: nonzero = the physics selection fixed at
-// compile time (PH_DEFAULT only).
-template<bool ADJ, bool DEP, uint32_t PHC = 0u>
-__global__ void __launch_bounds__(256, NBL_STEP_MIN_BLOCKS) k_step(const __grid_constant__ StepParams P, uint32_t it)
+// compile time (PH_DEFAULT only).  FINE: a fine mesh (1), a coarse one (0), or
+// what P.pass_empty says (-1).
+// Four resident blocks of 256 threads per SM (at most 64 registers): the
+// kernel waits for loads and instruction fetches, so warps in flight matter
+// more than the spills.
+template<bool ADJ, bool DEP, uint32_t PHC, int FINE>
+__global__ void __launch_bounds__(256, 4) k_step(const __grid_constant__ StepParams P, uint32_t it)
 {
 	__shared__ uint32_t s_counters[N_COUNTERS];
 	__shared__ float s_lane[DEP ? 256 : 1];
@@ -1011,7 +1012,7 @@ __global__ void __launch_bounds__(256, NBL_STEP_MIN_BLOCKS) k_step(const __grid_
 	// materials read from global memory: staged in shared memory as the
 	// batched kernel stages them, this kernel measured slower (-0.4 % on the
 	// grating scan, -1.5 % on the 1.2 M-triangle mesh)
-	step_iteration<ADJ, false, DEP, PHC>(P, none, it, lc, P.mats, s_rank + (threadIdx.x & ~31u), s_lane);
+	step_iteration<ADJ, false, DEP, PHC, FINE>(P, none, it, lc, P.mats, s_rank + (threadIdx.x & ~31u), s_lane);
 	flush_counters(P, lc, s_counters);
 }
 
@@ -1089,19 +1090,21 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 
 // The step kernel instantiation a run's parameters select: adjoint or not,
 // deposits or not, the default physics selection fixed at compile time or the
-// run-time word.
+// run-time word, fine or coarse mesh.
 static const void* step_kernel(const StepParams& p)
 {
 	const bool dep = p.dep || p.grid;
 	const bool fixed = p.phys == PH_DEFAULT;
 	if (p.adjoint) {
-		if (dep) return (const void*)k_step<true, true>;
-		if (fixed) return (const void*)k_step<true, false, PH_DEFAULT>;
-		return (const void*)k_step<true, false>;
+		if (dep) return (const void*)k_step<true, true, 0u, -1>;
+		if (!fixed) return (const void*)k_step<true, false, 0u, -1>;
+		if (p.pass_empty) return (const void*)k_step<true, false, PH_DEFAULT, 1>;
+		return (const void*)k_step<true, false, PH_DEFAULT, 0>;
 	}
-	if (dep) return (const void*)k_step<false, true>;
-	if (fixed) return (const void*)k_step<false, false, PH_DEFAULT>;
-	return (const void*)k_step<false, false>;
+	if (dep) return (const void*)k_step<false, true, 0u, -1>;
+	if (!fixed) return (const void*)k_step<false, false, 0u, -1>;
+	if (p.pass_empty) return (const void*)k_step<false, false, PH_DEFAULT, 1>;
+	return (const void*)k_step<false, false, PH_DEFAULT, 0>;
 }
 
 cudaError_t launch_step(const StepParams& p, uint32_t iteration, int grid, int block, cudaStream_t s)
@@ -1127,7 +1130,7 @@ cudaError_t step_binary_version(int device, int* version)
 	if (e != cudaSuccess)
 		return e;
 	cudaFuncAttributes a{};
-	e = cudaFuncGetAttributes(&a, k_step<false, false, PH_DEFAULT>);
+	e = cudaFuncGetAttributes(&a, k_step<false, false, PH_DEFAULT, 0>);
 	*version = a.binaryVersion;
 	return e;
 }

@@ -1,5 +1,12 @@
-"""A run's records do not depend on which lane flies a secondary: plain and
-batched runs, pools of different size and the adjoint's replay agree exactly.
+"""The step kernel's and the walk's variants against one another and the oracle.
+
+* Walks whose leaves hold lists longer than the 32 entries one pass of plane
+  tests covers, with slivers, grazing rays, rays in a triangle's plane and rays
+  that start outside the root cell: distance bits and triangle equal to the
+  oracle's walk, which tests every listed triangle.
+* A run's records do not depend on the empty leaves a fine mesh's walks pass
+  along, or on which lane flies a secondary.
+All comparisons are exact.
 """
 import numpy as np
 import pytest
@@ -7,6 +14,64 @@ import pytest
 import nebula_b200 as nb
 
 pytestmark = pytest.mark.gpu
+
+
+def _oracle_geometry(g):
+    from oracle import oracle as O
+    od, tr = g.export()
+    inf = g.info()
+    t11 = np.concatenate([np.stack([tr["material_in"], tr["material_out"]], 1).astype(np.float32),
+                          tr["r0"], tr["e1"], tr["e2"]], 1)
+    return O.Geometry(od, t11, inf["center"], inf["halfsize"], inf["max_extent"]), tr
+
+
+def _triangles(n, rng):
+    """Triangles of mixed size and shape in a 100 nm cube: ordinary ones,
+    slivers, coplanar pairs and axis-aligned ones."""
+    a = rng.uniform(-50, 50, (n, 3))
+    e1 = rng.standard_normal((n, 3)) * rng.choice([0.3, 5.0, 40.0], (n, 1))
+    e2 = rng.standard_normal((n, 3)) * rng.choice([0.3, 5.0, 40.0], (n, 1))
+    sliver = rng.random(n) < 0.2
+    e2[sliver] = e1[sliver] * rng.uniform(0.5, 1.5, (sliver.sum(), 1)) + rng.standard_normal((sliver.sum(), 3)) * 1e-3
+    flat = rng.random(n) < 0.2
+    e1[flat, 2] = e2[flat, 2] = 0.0
+    a[flat, 2] = np.round(a[flat, 2] / 25) * 25
+    mats = rng.choice([0, 1, -123], (n, 2))
+    return np.hstack([mats, a, a + e1, a + e2])
+
+
+@pytest.mark.parametrize("n_tri", [1, 31, 32, 33, 64, 65, 300])
+def test_walk_equals_oracle_for_any_list_length(n_tri):
+    rng = np.random.default_rng(n_tri)
+    g = nb.Geometry.from_triangles(_triangles(n_tri, rng), max_depth=2, split_count=400)
+    og, tr = _oracle_geometry(g)
+    n = 200_000
+    pos = rng.uniform(-60, 60, (n, 3))
+    d = rng.standard_normal((n, 3))
+    # a third of the rays start near a triangle's plane and run almost along it
+    k = rng.integers(0, len(tr), n)
+    e1, e2, r0 = (tr[f][k].astype(np.float64) for f in ("e1", "e2", "r0"))
+    nrm = np.cross(e1, e2)
+    nrm /= np.maximum(np.linalg.norm(nrm, axis=1, keepdims=True), 1e-30)
+    graze = np.arange(n) % 3 == 0
+    w = rng.standard_normal((n, 2))
+    along = w[:, :1] * e1 + w[:, 1:] * e2 + nrm * rng.choice([0, 1e-7, 1e-4, 1e-2], (n, 1))
+    start = r0 + rng.uniform(-1, 2, (n, 1)) * e1 + rng.uniform(-1, 2, (n, 1)) * e2 + nrm * rng.choice([0, 1e-6, 1e-3], (n, 1))
+    d[graze], pos[graze] = along[graze], start[graze]
+    d[np.arange(n) % 7 == 1, 0] = 0.0
+    outside = np.arange(n) % 11 == 5
+    pos[outside] *= 30.0
+    d[outside] = -pos[outside] + rng.standard_normal((outside.sum(), 3))
+    d /= np.maximum(np.linalg.norm(d, axis=1, keepdims=True), 1e-30)
+    pos, d = pos.astype(np.float32), d.astype(np.float32)
+    dist = np.where(rng.random(n) < 0.5, rng.exponential(5.0, n), 1e4).astype(np.float32)
+    ignore_tri = np.where(rng.random(n) < 0.2, k, -1).astype(np.int32)
+    ignore_mat = rng.choice([0, 1, -123], n).astype(np.int32)
+    gd, gt = g.ray_query(pos, d, dist, ignore_tri, ignore_mat)
+    cd, ct = og.propagate(pos, d, dist, ignore_tri, ignore_mat)
+    assert np.array_equal(gt, ct), int((gt != ct).sum())
+    assert np.array_equal(gd.view(np.uint32), cd.view(np.uint32))
+    assert n_tri < 31 or (gt >= 0).any()
 
 
 def _sorted(rec):
@@ -21,6 +86,27 @@ def _records(g, mats, pri, **kw):
     sim.close()
     assert c["primaries_started"] + c["spawned"] == c["detected"] + c["terminated"]
     return rec, c
+
+
+def test_fine_mesh_equals_batch_and_other_budgets(inputs):
+    """The batch passes no empty leaves along, the plain run on a fine mesh does."""
+    from nebula_b200.synth import geometry, primaries
+    mats = [nb.Material.load(inputs["si.nmat"]), nb.Material.load(inputs["pmma.nmat"])]
+    rows = geometry.rough_grating(n_lines=4, line_length=100.0, vertex_spacing=0.25)
+    g = nb.Geometry.from_triangles(rows, max_depth=12, split_count=16)
+    assert g.info()["n_octree"] >= 1 << 20
+    pri = primaries.raster_scan(16, 16, 20, 0.5, 300.0, 40.0, spot_sigma=1.0, seed=3)
+    one, c1 = _records(g, mats, pri)
+    long, c2 = _records(g, mats, pri, walk_cells=1 << 10)
+    batch = nb.Batch([g], mats, capacity=1 << 16, record_capacity=1 << 20)
+    batch.set_jobs([(0, 77, pri)])
+    batch.run()
+    rec, _ = batch.records()
+    batch.close()
+    assert c1["walk_resumes"] > 0 and c1["flights"] == c2["flights"]
+    assert len(one) > 0
+    assert np.array_equal(_sorted(one), _sorted(long))
+    assert np.array_equal(_sorted(one), _sorted(rec))
 
 
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 65])
