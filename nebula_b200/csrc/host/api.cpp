@@ -79,6 +79,14 @@ struct nbl_sim {
 	uint64_t pri_cap = 0, n_pri = 0;
 	StepParams sp{};
 	int grid = 0, block = 256;
+	int grid_for[2] = { 0, 0 };             // blocks of the step kernel for many and for few electrons
+	// Runs with at most this many primaries take the step kernel with three
+	// blocks per SM: 10 k slab primaries 1.96 against 2.27 ms, 4 001 at 15 keV
+	// 10.6 / 11.9, 50 k with deposits 3.47 / 3.80, 205 k Kieft-Bosch grating
+	// 3.95 / 4.13; at 300 k slab primaries still 10.94 / 11.17, but an adjoint
+	// scan of 410 k takes 35.3 against 34.8 and 922 k on the grating 27.0
+	// against 26.5 (four blocks second)
+	static constexpr uint64_t FEW_PRIMARIES = 1u << 18;
 	uint32_t graph_iters = 24;
 	uint64_t iteration = 0;
 	cudaGraphExec_t graph = nullptr;
@@ -167,6 +175,8 @@ struct nbl_sim {
 
 	void build_graph()
 	{
+		sp.few = n_pri <= FEW_PRIMARIES ? 1 : 0;
+		grid = params.grid_size ? (int)params.grid_size : grid_for[sp.few];
 		if (graph) {
 			cudaGraphExecDestroy(graph);
 			graph = nullptr;
@@ -975,7 +985,9 @@ nbl_status nbl_sim_create(const nbl_geometry* g, nbl_material* const* materials,
 		sp.max_events = params->max_events ? params->max_events : (1u << 22);
 		require(sp.max_events < (1u << 24), "max_events must be < 2^24");
 		sp.adjoint = adj ? 1 : 0;
-		s->grid = params->grid_size ? (int)params->grid_size : step_grid_size(s->device, s->block, sp);
+		for (sp.few = 0; sp.few < 2; ++sp.few)
+			s->grid_for[sp.few] = step_grid_size(s->device, s->block, sp);
+		sp.few = 0;
 		s->ensure_primary_capacity(1024);
 		sp.n_primaries = 0;
 		s->reset_device_state();

@@ -105,6 +105,7 @@ struct StepParams {
 	int32_t gn[3];
 	uint32_t walk_cells;      // leaf cells a flight's walk takes per iteration before it continues in the next
 	int32_t pass_empty;       // empty leaves passed before each of them (0 or PASS_EMPTY)
+	int32_t few;              // few electrons in flight: the step kernel with more registers per thread
 };
 
 // Work-function sign of a primary for material m (0 or 1): +1 or -1 from a

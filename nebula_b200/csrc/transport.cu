@@ -995,11 +995,13 @@ __device__ __forceinline__ void flush_counters(const StepParams& P, LocalCounter
 // none of their code).  PHC: nonzero = the physics selection fixed at
 // compile time (PH_DEFAULT only).  FINE: a fine mesh (1), a coarse one (0), or
 // what P.pass_empty says (-1).
-// Four resident blocks of 256 threads per SM (at most 64 registers): the
-// kernel waits for loads and instruction fetches, so warps in flight matter
-// more than the spills.
-template<bool ADJ, bool DEP, uint32_t PHC, int FINE>
-__global__ void __launch_bounds__(256, 4) k_step(const __grid_constant__ StepParams P, uint32_t it)
+// BLOCKS: resident blocks of 256 threads per SM.  Four (64 registers a thread,
+// some spilled) where the chip is full: the kernel waits for loads and
+// instruction fetches, and warps in flight matter more than the spills.  Three
+// (80 registers, none spilled) for runs that never fill it, whose time is the
+// latency of one chunk after the other.
+template<bool ADJ, bool DEP, uint32_t PHC, int FINE, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_step(const __grid_constant__ StepParams P, uint32_t it)
 {
 	__shared__ uint32_t s_counters[N_COUNTERS];
 	__shared__ float s_lane[DEP ? 256 : 1];
@@ -1090,21 +1092,27 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 
 // The step kernel instantiation a run's parameters select: adjoint or not,
 // deposits or not, the default physics selection fixed at compile time or the
-// run-time word, fine or coarse mesh.
+// run-time word, fine or coarse mesh, few electrons or many.
+template<bool ADJ, bool DEP, uint32_t PHC, int FINE>
+static const void* step_kernel_for(const StepParams& p)
+{
+	return p.few ? (const void*)k_step<ADJ, DEP, PHC, FINE, 3> : (const void*)k_step<ADJ, DEP, PHC, FINE, 4>;
+}
+
 static const void* step_kernel(const StepParams& p)
 {
 	const bool dep = p.dep || p.grid;
 	const bool fixed = p.phys == PH_DEFAULT;
 	if (p.adjoint) {
-		if (dep) return (const void*)k_step<true, true, 0u, -1>;
-		if (!fixed) return (const void*)k_step<true, false, 0u, -1>;
-		if (p.pass_empty) return (const void*)k_step<true, false, PH_DEFAULT, 1>;
-		return (const void*)k_step<true, false, PH_DEFAULT, 0>;
+		if (dep) return (const void*)k_step<true, true, 0u, -1, 4>;
+		if (!fixed) return (const void*)k_step<true, false, 0u, -1, 4>;
+		if (p.pass_empty) return (const void*)k_step<true, false, PH_DEFAULT, 1, 4>;
+		return step_kernel_for<true, false, PH_DEFAULT, 0>(p);
 	}
-	if (dep) return (const void*)k_step<false, true, 0u, -1>;
-	if (!fixed) return (const void*)k_step<false, false, 0u, -1>;
-	if (p.pass_empty) return (const void*)k_step<false, false, PH_DEFAULT, 1>;
-	return (const void*)k_step<false, false, PH_DEFAULT, 0>;
+	if (dep) return step_kernel_for<false, true, 0u, -1>(p);
+	if (!fixed) return step_kernel_for<false, false, 0u, -1>(p);
+	if (p.pass_empty) return step_kernel_for<false, false, PH_DEFAULT, 1>(p);
+	return step_kernel_for<false, false, PH_DEFAULT, 0>(p);
 }
 
 cudaError_t launch_step(const StepParams& p, uint32_t iteration, int grid, int block, cudaStream_t s)
@@ -1130,7 +1138,7 @@ cudaError_t step_binary_version(int device, int* version)
 	if (e != cudaSuccess)
 		return e;
 	cudaFuncAttributes a{};
-	e = cudaFuncGetAttributes(&a, k_step<false, false, PH_DEFAULT, 0>);
+	e = cudaFuncGetAttributes(&a, k_step<false, false, PH_DEFAULT, 0, 4>);
 	*version = a.binaryVersion;
 	return e;
 }

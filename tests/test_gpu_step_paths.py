@@ -4,8 +4,9 @@
   tests covers, with slivers, grazing rays, rays in a triangle's plane and rays
   that start outside the root cell: distance bits and triangle equal to the
   oracle's walk, which tests every listed triangle.
-* A run's records do not depend on the empty leaves a fine mesh's walks pass
-  along, or on which lane flies a secondary.
+* A run's records do not depend on which step kernel its size selects (few
+  primaries or many), on the empty leaves a fine mesh's walks pass along, or on
+  which lane flies a secondary.
 All comparisons are exact.
 """
 import numpy as np
@@ -86,6 +87,19 @@ def _records(g, mats, pri, **kw):
     sim.close()
     assert c["primaries_started"] + c["spawned"] == c["detected"] + c["terminated"]
     return rec, c
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1000])
+def test_few_and_many_primaries_give_the_same_records(inputs, n):
+    from nebula_b200.synth import primaries
+    g = nb.Geometry.from_tri_file(inputs["slab.tri"])
+    m = nb.Material.load(inputs["si.nmat"])
+    total = (1 << 19) + 1
+    pri = primaries.point_beam(total, energy=150.0)
+    pri["px"] = np.arange(total)
+    few, _ = _records(g, [m], pri[:n], capacity=1 << 16)
+    many, _ = _records(g, [m], pri, capacity=1 << 18)
+    assert np.array_equal(_sorted(few), _sorted(many[many["px"] < n]))
 
 
 def test_fine_mesh_equals_batch_and_other_budgets(inputs):
