@@ -343,41 +343,44 @@ __device__ __forceinline__ bool flight_begin(const StepParams& P, const DevGeome
 	return true;
 }
 
-// Free flight of an electron whose flight_begin passed: free-path sampling,
-// octree walk, move.  Returns the queue of the event the flight ends in, -1
-// when the electron is terminated, or EV_WALK when the walk reached the run's
-// per-iteration cell budget (`fr` then holds where it stands).  With `resume`,
-// the flight stored in `fr` continues (its checks, event count and random
-// draws are behind it).  A flight in vacuum that hits nothing ends without an
+// Free path of an electron whose flight_begin passed: `fr` receives the
+// flight's length, what ends it and the walk's start.
+template<bool ADJ>
+__device__ __forceinline__ void flight_sample(const RunView& rv, const Electron& p, int mat, uint32_t event,
+	uint32_t stream_tag, uint64_t lineage, FlightResume& fr, const DevMaterial* mats)
+{
+	fr.hop = 0;
+	fr.type = 0;
+	fr.dist = rv.geom->max_extent;
+	if (mat >= 0) {
+		const DevMaterial* const m = mats + mat;
+		PhiloxStream r;
+		r.init(rv.key, event, 0u, stream_tag, lineage);
+		float u[4], mu;
+		r.block(0, u);
+		const float pe = sample_path(m->el_imfp, m->el_scale, p.E, u[0], mu);
+		const float pi = sample_path(m->in_imfp, m->in_scale, p.E, u[1], mu);
+		fr.dist = __int_as_float(0x7f800000);
+		if (pe < fr.dist) { fr.dist = pe; fr.type = 2; }
+		if (pi < fr.dist) { fr.dist = pi; fr.type = 1; }
+	}
+	fr.w = walk_start(p.pos.x, p.pos.y, p.pos.z, fr.dist);
+}
+
+// The flight in `fr`, sampled or continued: octree walk and move.  Returns the
+// queue of the event the flight ends in, -1 when the electron is terminated, or
+// EV_WALK when the walk reached the run's per-iteration cell budget (`fr` then
+// holds where it stands).  A flight in vacuum that hits nothing ends without an
 // event and is repeated (`repeats`; the next one leaves the domain as a rule,
 // else it is queued as a walk that has not started, four flights in all).
-// Mirrors cpu_driver::init / kernels::init
+// Mirrors, with flight_begin and flight_sample, cpu_driver::init / kernels::init
 // (drivers/cpu/cpu_driver.inl:74-130, drivers/gpu/gpu_driver.inl:403-480).
 template<bool ADJ>
-__device__ __forceinline__ int free_flight(const StepParams& P, const RunView& rv, Electron& p, int mat, int& last_tri,
-	uint32_t& event, uint32_t stream_tag, uint64_t lineage, float* sc, LocalCounters& lc, const float* dbar,
-	FlightResume& fr, bool resume, const DevMaterial* mats, int pass_empty, int& repeats)
+__device__ __forceinline__ int flight_walk(const StepParams& P, const RunView& rv, Electron& p, int mat, int& last_tri,
+	uint32_t& event, float* sc, LocalCounters& lc, const float* dbar, FlightResume& fr, const DevMaterial* mats,
+	int pass_empty, int& repeats)
 {
 	const DevGeometry& G = *rv.geom;
-	const DevMaterial* const m = mats + mat;              // read for mat >= 0 only
-	float mu_el = 0.0f, mu_in = 0.0f;
-	if (!resume) {
-		fr.hop = 0;
-		fr.type = 0;
-		fr.dist = G.max_extent;
-		if (mat >= 0) {
-			PhiloxStream r;
-			r.init(rv.key, event, 0u, stream_tag, lineage);
-			float u[4];
-			r.block(0, u);
-			const float pe = sample_path(m->el_imfp, m->el_scale, p.E, u[0], mu_el);
-			const float pi = sample_path(m->in_imfp, m->in_scale, p.E, u[1], mu_in);
-			fr.dist = __int_as_float(0x7f800000);
-			if (pe < fr.dist) { fr.dist = pe; fr.type = 2; }
-			if (pi < fr.dist) { fr.dist = pi; fr.type = 1; }
-		}
-		fr.w = walk_start(p.pos.x, p.pos.y, p.pos.z, fr.dist);
-	}
 	const V3 d = vnormalised(p.dir);
 	float idist;
 	const int hit = propagate_cells(G, fr.w, d.x, d.y, d.z, fr.dist, last_tri, mat, idist, (int)P.walk_cells,
@@ -389,11 +392,10 @@ __device__ __forceinline__ int free_flight(const StepParams& P, const RunView& r
 		// score of the flight: density mu_k exp(-(mu_in+mu_el) d) of the
 		// chosen event k at distance d, or survival exp(-(mu_in+mu_el) d)
 		// when a boundary cuts the flight; derivative w.r.t. the scales
-		if (resume) {
-			// the inverse mean free paths the flight was sampled with
-			mu_el = imfp_at(m->el_imfp, m->el_scale, p.E);
-			mu_in = imfp_at(m->in_imfp, m->in_scale, p.E);
-		}
+		// (the inverse mean free paths are those it was sampled with)
+		const DevMaterial* const m = mats + mat;
+		const float mu_el = imfp_at(m->el_imfp, m->el_scale, p.E);
+		const float mu_in = imfp_at(m->in_imfp, m->in_scale, p.E);
 		const float travel = hit >= 0 ? idist : fr.dist;
 		const float in_k = (hit < 0 && fr.type == 1) ? 1.0f : 0.0f;
 		const float el_k = (hit < 0 && fr.type == 2) ? 1.0f : 0.0f;
@@ -634,15 +636,36 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 	const Queue* qout = P.q[(it + 1u) & 1u];
 
 	const uint32_t lane = threadIdx.x & 31u;
-	// Warps take 32 items at a time from a counter in the read slot (zeroed
-	// two iterations ago, untouched since), so the iteration ends when the
-	// work does rather than when the slowest warp's fixed share does.
+	// Work is handed out from a counter in the read slot (zeroed two
+	// iterations ago, untouched since), so the iteration ends when the work
+	// does rather than when the slowest warp's fixed share does.  A block
+	// claims one item per thread and its warps go through a chunk's phases
+	// (state, event, sampling, walk, append) together: the phases' code is 74 KB,
+	// far more than the instruction caches next to the schedulers, and warps
+	// that stand in the same phase fetch it once.  That takes the stalls for
+	// instructions from 3.0 to 0.5 per issued one for less than that in waits
+	// at the barriers: grating 160 x 160 x 100 68.2 -> 65.8 ms, slab 300 k 11.0
+	// -> 10.4, 10 k 2.05 -> 1.82, batch of 20 jobs 23.7 -> 21.5; blocks of 128
+	// and 512 threads gain less.  On a fine mesh, whose walks wait for loads of
+	// very different latency, the barriers cost more than they save (64.3 ->
+	// 65.2 ms on the rough lines): there each warp claims its own chunk.
+	constexpr bool TOGETHER = FINE != 1;
+	const auto phase = [] { if (TOGETHER) __syncthreads(); };
 	uint32_t* const work = P.ctrl + rs * SLOT_WORDS + SLOT_WORK;
+	__shared__ uint32_t s_base;
 	uint32_t base = 0u;
-	if (lane == 0u) base = atomicAdd(work, 32u);
-	base = __shfl_sync(0xFFFFFFFFu, base, 0);
+	if (TOGETHER) {
+		if (threadIdx.x == 0u) s_base = atomicAdd(work, blockDim.x);
+		__syncthreads();
+		base = s_base;
+	} else {
+		if (lane == 0u) base = atomicAdd(work, 32u);
+		base = __shfl_sync(0xFFFFFFFFu, base, 0);
+	}
 
 	for (; base < total; ) {
+		if (TOGETHER)
+			base += threadIdx.x & ~31u;
 		const uint32_t item = base + lane;
 		// item kinds: the queues EV_BOUNDARY .. EV_WALK, then K_RING (a
 		// secondary drained from the spill ring) and K_PRIMARY (a new primary)
@@ -721,6 +744,7 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 			dbar[1] = fm(P.wstep, wsign(rv.key, stream_tag, 1));
 		}
 
+		phase();
 		// interaction that ended the previous flight
 		int status = (kind >= 0) ? ST_RUNNING : ST_TERMINATED;
 		bool spawn = false;
@@ -904,12 +928,21 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 		}
 
 		// next free flight (or the rest of a walk cut short last iteration)
-		int qtype = -1, repeats = 0;
+		phase();
 		if (kind == EV_WALK)
 			load_resume(qin[EV_WALK], qi, fr);
+		else if (flying)
+			flight_sample<ADJ>(rv, p, mat, event, stream_tag, lineage, fr, mats);
+		phase();
+		int qtype = -1, repeats = 0;
 		if (flying)
-			qtype = free_flight<ADJ>(P, rv, p, mat, last_tri, event, stream_tag, lineage, sc, lc,
-				wshift ? dbar : nullptr, fr, kind == EV_WALK, mats, pass_empty, repeats);
+			qtype = flight_walk<ADJ>(P, rv, p, mat, last_tri, event, sc, lc, wshift ? dbar : nullptr, fr, mats, pass_empty,
+				repeats);
+		// the block's next chunk (every warp has read the last claim: the
+		// phases since then are barriers)
+		if (TOGETHER && threadIdx.x == 0u)
+			s_base = atomicAdd(work, blockDim.x);
+		phase();
 		const unsigned ended = __ballot_sync(0xFFFFFFFFu, flying && qtype < 0);
 		if (ended) {
 			if (lane == (uint32_t)CNT_TERMINATED)
@@ -923,10 +956,10 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 		if (repeats)
 			atomicAdd(lc.c + CNT_FLIGHTS, (uint32_t)repeats);
 		{
-			// the warp's next chunk is claimed (lane 5) together with the
+			// a warp's own next chunk is claimed (lane 5) together with the
 			// queue slots (lanes 0-4): one atomic round trip for both
 			uint32_t next = 0u;
-			if (lane == 5u)
+			if (!TOGETHER && lane == 5u)
 				next = atomicAdd(work, 32u);
 			const uint32_t slot = warp_reserve5(cw, qtype);
 			if (qtype >= 0 && slot >= P.qcap)
@@ -945,7 +978,7 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 						store_resume(qout[t], slot, fr);
 				}
 			}
-			base = __shfl_sync(0xFFFFFFFFu, next, 5);
+			base = TOGETHER ? s_base : __shfl_sync(0xFFFFFFFFu, next, 5);
 		}
 	}
 	return true;
