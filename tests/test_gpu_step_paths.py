@@ -142,3 +142,27 @@ def test_secondaries_flown_in_ended_lanes(inputs, n):
     rec, _ = batch.records()
     batch.close()
     assert np.array_equal(_sorted(ref), _sorted(rec))
+
+
+def test_reused_simulation_equals_fresh_ones(inputs):
+    """Runs of one simulation with the same and with other counts, seeds and
+    offsets (its launch graph is kept while they are the same)."""
+    from nebula_b200.synth import primaries
+    g = nb.Geometry.from_tri_file(inputs["slab.tri"])
+    m = nb.Material.load(inputs["si.nmat"])
+    sim = nb.Simulation(g, [m], capacity=1 << 12, seed=77)
+    for seed, first, n, energy in ((77, 0, 200, 500.0), (77, 0, 200, 300.0), (78, 0, 200, 300.0), (78, 5, 200, 300.0),
+                                   (78, 5, 201, 300.0), (78, 5, 5000, 300.0), (77, 0, 200, 500.0)):
+        pri = primaries.point_beam(n, energy=energy)
+        sim.reset()
+        sim.set_seed(seed)
+        sim.set_primary_offset(first)
+        sim.push(pri)
+        sim.run()
+        fresh = nb.Simulation(g, [m], capacity=1 << 12, seed=seed)
+        fresh.set_primary_offset(first)
+        fresh.push(pri)
+        fresh.run()
+        assert np.array_equal(_sorted(sim.flush_detected()), _sorted(fresh.flush_detected()))
+        fresh.close()
+    sim.close()
