@@ -166,3 +166,29 @@ def test_reused_simulation_equals_fresh_ones(inputs):
         assert np.array_equal(_sorted(sim.flush_detected()), _sorted(fresh.flush_detected()))
         fresh.close()
     sim.close()
+
+
+@pytest.mark.parametrize("n", [116_508, 116_509, 150_001])
+def test_large_pageable_push_equals_pinned(inputs, n):
+    """Pushes of 4 MiB and more (116 509 records) go through staging threads;
+    from page-locked memory, or in small parts, they are copied directly."""
+    import torch
+    from nebula_b200.synth import primaries
+    g = nb.Geometry.from_tri_file(inputs["slab.tri"])
+    m = nb.Material.load(inputs["si.nmat"])
+    pri = primaries.point_beam(n, energy=60.0)
+    pri["px"] = np.arange(n)
+    pri["pos"][:, 0] = np.random.default_rng(n).uniform(-300, 300, n)
+    pinned = torch.empty(n * 36, dtype=torch.uint8, pin_memory=True).numpy().view(nb.PRI_DTYPE)
+    pinned[:] = pri
+    whole, _ = _records(g, [m], pri, capacity=1 << 16)
+    direct, _ = _records(g, [m], pinned, capacity=1 << 16)
+    sim = nb.Simulation(g, [m], capacity=1 << 16, seed=77)
+    for part in np.array_split(pri, 5):
+        sim.push(part)
+    sim.run()
+    parts = sim.flush_detected()
+    sim.close()
+    assert len(whole) > 0
+    assert np.array_equal(_sorted(whole), _sorted(direct))
+    assert np.array_equal(_sorted(whole), _sorted(parts))
