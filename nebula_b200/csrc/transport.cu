@@ -12,7 +12,9 @@
 // electrons are in flight, at most `ramp` per iteration).  Each item performs
 // the interaction that ended its previous free flight, then its next free
 // flight (free-path sampling + octree walk), and is appended to the next
-// iteration's queue for the event that flight ended in.  A walk stops after
+// iteration's queue for the event that flight ended in.  A lane whose electron
+// ended flies a secondary of its warp instead; the flight queue takes those
+// that find no lane.  A walk stops after
 // `walk_cells` leaf cells (default 1); an unfinished one is appended to the
 // continued-walk queue with its exact state and goes on in the next
 // iteration, so a warp never waits on its lane with the longest walk.  Queues are
@@ -1055,13 +1057,16 @@ __global__ void __launch_bounds__(256, BLOCKS) k_step(const __grid_constant__ St
 // cooperative launch).  Arrival counter + generation word; waiting is bounded
 // (2^22 polls, a few seconds; one iteration takes milliseconds); on timeout,
 // or if any block already timed out, it records the error and returns false
-// so every block leaves.
+// so every block leaves.  The waiting blocks read the generation with plain
+// loads: as atomics, hundreds of them queued up in front of the arrivals.
 __device__ __forceinline__ bool grid_barrier(const BatchParams& B)
 {
 	__shared__ int s_ok;
 	__syncthreads();
 	if (threadIdx.x == 0) {
-		const unsigned gen0 = atomicAdd(B.bar_gen, 0u);
+		const volatile unsigned* const gen = B.bar_gen;
+		const volatile unsigned* const err = B.err;
+		const unsigned gen0 = *gen;
 		__threadfence();
 		const unsigned arrived = atomicAdd(B.bar_count, 1u) + 1u;
 		int ok = 1;
@@ -1071,14 +1076,14 @@ __device__ __forceinline__ bool grid_barrier(const BatchParams& B)
 			atomicAdd(B.bar_gen, 1u);
 		} else {
 			unsigned polls = 0;
-			while (atomicAdd(B.bar_gen, 0u) == gen0) {
-				if (atomicAdd(B.err, 0u)) { ok = 0; break; }
-				__nanosleep(64);
+			while (*gen == gen0) {
+				if (*err) { ok = 0; break; }
+				__nanosleep(32);
 				if (++polls > (1u << 22)) { atomicOr(B.err, 1u); ok = 0; break; }
 			}
 		}
 		__threadfence();
-		s_ok = ok && atomicAdd(B.err, 0u) == 0u;
+		s_ok = ok && *err == 0u;
 	}
 	__syncthreads();
 	return s_ok != 0;
