@@ -66,31 +66,34 @@ HostTable copy_table(const nbl_table& t)
 // Host to device copies of pageable memory.  The driver stages such a copy
 // through one thread (some 10 GB/s); here four threads copy blocks of it into
 // page-locked buffers and send them on from there (some 18 GB/s: 92 MB of
-// primaries 9.4 -> 5.2 ms; 1 MB blocks take 3.6 but their buffers longer to make).
+// primaries 9.4 -> 5.2 ms; 128 KiB blocks 6.3, 1 MiB blocks 3.6, but the
+// larger the buffers the longer the first push takes to make them).
 namespace {
 
 class PageableCopy {
 public:
-	static constexpr size_t MIN_BYTES = (size_t)4 << 20;   // below, starting the threads is not worth it
+	// (below, the buffers cost a simulation's first push more than they save it)
+	static constexpr size_t MIN_BYTES = (size_t)16 << 20;
 	static constexpr int LANES = 4;
 	static constexpr size_t BLOCK = (size_t)256 << 10;
-	static constexpr size_t BUFFER_BYTES = 2 * LANES * BLOCK;
 
 	~PageableCopy()
 	{
 		for (Lane& l : lanes)
 			for (cudaEvent_t e : l.sent)
 				if (e) cudaEventDestroy(e);
+		if (buffer) cudaFreeHost(buffer);
 	}
 
-	// Enqueues on `stream` and returns when all of it has arrived.  `buffer`:
-	// BUFFER_BYTES of page-locked memory that nothing else uses meanwhile.
-	void run(void* dst, const void* src, size_t bytes, char* buffer, int device, cudaStream_t stream)
+	// Enqueues on `stream` and returns when all of it has arrived.
+	void run(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream)
 	{
+		if (!buffer)
+			CU(cudaMallocHost(&buffer, 2 * LANES * BLOCK));
 		for (Lane& l : lanes)
 			for (cudaEvent_t& e : l.sent)
 				if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-		const auto part = [=](int lane) { work(lane, dst, src, bytes, buffer, device, stream); };
+		const auto part = [=](int lane) { work(lane, dst, src, bytes, device, stream); };
 		std::thread helpers[LANES - 1];
 		int started = 0;
 		try {
@@ -116,9 +119,10 @@ private:
 		cudaError_t err = cudaSuccess;
 	};
 	Lane lanes[LANES];
+	char* buffer = nullptr;       // 2 MiB, made at the first copy
 
 	// blocks lane, lane + LANES, ... through the lane's two buffers in turn
-	void work(int lane, void* dst, const void* src, size_t bytes, char* buffer, int device, cudaStream_t stream)
+	void work(int lane, void* dst, const void* src, size_t bytes, int device, cudaStream_t stream)
 	{
 		Lane& l = lanes[lane];
 		l.err = cudaSetDevice(device);
@@ -179,11 +183,7 @@ struct nbl_sim {
 	uint32_t record_growth = 0;             // most records one graph has added
 	uint32_t* pinned_ctrl = nullptr;        // control slot, record count, then the counters
 	static constexpr size_t PINNED_COUNTERS_OFFSET = ((SLOT_WORDS + 4) * sizeof(uint32_t) + 7) & ~(size_t)7;
-	// (then, page-aligned, the staging buffers of pageable pushes)
-	static constexpr size_t PINNED_STAGING_OFFSET =
-		(PINNED_COUNTERS_OFFSET + N_COUNTERS * sizeof(unsigned long long) + 4095) & ~(size_t)4095;
-	static constexpr size_t PINNED_BYTES = PINNED_STAGING_OFFSET + PageableCopy::BUFFER_BYTES;
-	char* staging() { return reinterpret_cast<char*>(pinned_ctrl) + PINNED_STAGING_OFFSET; }
+	static constexpr size_t PINNED_BYTES = PINNED_COUNTERS_OFFSET + N_COUNTERS * sizeof(unsigned long long);
 	unsigned long long* pinned_counters()
 	{
 		return reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(pinned_ctrl) + PINNED_COUNTERS_OFFSET);
@@ -1111,7 +1111,7 @@ static void push_common(nbl_sim* s, const void* src, int64_t n, cudaMemcpyKind k
 		staged = a.type == cudaMemoryTypeUnregistered;
 	}
 	if (staged) {
-		s->pageable.run(dst, src, bytes, s->staging(), s->device, s->stream);
+		s->pageable.run(dst, src, bytes, s->device, s->stream);
 	} else {
 		CU(cudaMemcpyAsync(dst, src, bytes, kind, s->stream));
 		CU(cudaStreamSynchronize(s->stream));

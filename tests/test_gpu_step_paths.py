@@ -168,9 +168,9 @@ def test_reused_simulation_equals_fresh_ones(inputs):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [116_508, 116_509, 150_001])
+@pytest.mark.parametrize("n", [466_033, 466_034, 500_001])
 def test_large_pageable_push_equals_pinned(inputs, n):
-    """Pushes of 4 MiB and more (116 509 records) go through staging threads;
+    """Pushes of 16 MiB and more (466 034 records) go through staging threads;
     from page-locked memory, or in small parts, they are copied directly."""
     import torch
     from nebula_b200.synth import primaries
