@@ -61,7 +61,7 @@ BYTES_PER_EVENT = 96   # 48-byte electron state read + written per event
 # exceeds the 96 algorithmic bytes because a flight whose walk continues in
 # the next iteration reads and writes its state again, plus 32 bytes of walk
 # state each way.
-DRAM_BYTES_PER_EVENT = 141.2
+DRAM_BYTES_PER_EVENT = 113.1
 
 
 def measured_peaks():
