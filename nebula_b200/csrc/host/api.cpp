@@ -2,6 +2,7 @@
 // debug entry points.  See include/nebula_b200.h for the contract.
 #include "internal.hpp"
 #include "device.hpp"
+#include "pageable.hpp"
 
 #include <cuda_runtime.h>
 #include "../device/rng.cuh"
@@ -12,8 +13,6 @@
 #include <sstream>
 #include <algorithm>
 #include <memory>
-#include <system_error>
-#include <thread>
 
 using namespace nbl;
 
@@ -63,86 +62,6 @@ HostTable copy_table(const nbl_table& t)
 }  // namespace nbl
 
 /* ======================================================================= */
-// Host to device copies of pageable memory.  The driver stages such a copy
-// through one thread (some 10 GB/s); here four threads copy blocks of it into
-// page-locked buffers and send them on from there (some 18 GB/s: 92 MB of
-// primaries 9.4 -> 5.2 ms; 128 KiB blocks 6.3, 1 MiB blocks 3.6, but the
-// larger the buffers the longer the first push takes to make them).
-namespace {
-
-class PageableCopy {
-public:
-	// (below, the buffers cost a simulation's first push more than they save it)
-	static constexpr size_t MIN_BYTES = (size_t)16 << 20;
-	static constexpr int LANES = 4;
-	static constexpr size_t BLOCK = (size_t)256 << 10;
-
-	~PageableCopy()
-	{
-		for (Lane& l : lanes)
-			for (cudaEvent_t e : l.sent)
-				if (e) cudaEventDestroy(e);
-		if (buffer) cudaFreeHost(buffer);
-	}
-
-	// Enqueues on `stream` and returns when all of it has arrived.
-	void run(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream)
-	{
-		if (!buffer)
-			CU(cudaMallocHost(&buffer, 2 * LANES * BLOCK));
-		for (Lane& l : lanes)
-			for (cudaEvent_t& e : l.sent)
-				if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-		const auto part = [=](int lane) { work(lane, dst, src, bytes, device, stream); };
-		std::thread helpers[LANES - 1];
-		int started = 0;
-		try {
-			for (; started < LANES - 1; ++started)
-				helpers[started] = std::thread(part, started + 1);
-		} catch (const std::system_error&) {
-			// no more threads: their blocks are copied here
-		}
-		part(0);
-		for (int i = started + 1; i < LANES; ++i)
-			part(i);
-		for (int i = 0; i < started; ++i)
-			helpers[i].join();
-		const cudaError_t e = cudaStreamSynchronize(stream);
-		for (const Lane& l : lanes)
-			CU(l.err);
-		CU(e);
-	}
-
-private:
-	struct Lane {
-		cudaEvent_t sent[2] = { nullptr, nullptr };
-		cudaError_t err = cudaSuccess;
-	};
-	Lane lanes[LANES];
-	char* buffer = nullptr;       // 2 MiB, made at the first copy
-
-	// blocks lane, lane + LANES, ... through the lane's two buffers in turn
-	void work(int lane, void* dst, const void* src, size_t bytes, int device, cudaStream_t stream)
-	{
-		Lane& l = lanes[lane];
-		l.err = cudaSetDevice(device);
-		int turn = 0;
-		for (size_t at = (size_t)lane * BLOCK; at < bytes && l.err == cudaSuccess; at += LANES * BLOCK, turn ^= 1) {
-			const size_t n = std::min(BLOCK, bytes - at);
-			char* const b = buffer + (2 * lane + turn) * BLOCK;
-			// the buffer's last block has left it (no record yet: nothing to wait for)
-			l.err = cudaEventSynchronize(l.sent[turn]);
-			if (l.err != cudaSuccess) break;
-			std::memcpy(b, static_cast<const char*>(src) + at, n);
-			l.err = cudaMemcpyAsync(static_cast<char*>(dst) + at, b, n, cudaMemcpyHostToDevice, stream);
-			if (l.err != cudaSuccess) break;
-			l.err = cudaEventRecord(l.sent[turn], stream);
-		}
-	}
-};
-
-}  // namespace
-
 /* simulation object                                                        */
 struct nbl_sim {
 	PageableCopy pageable;
@@ -1110,8 +1029,8 @@ static void push_common(nbl_sim* s, const void* src, int64_t n, cudaMemcpyKind k
 			cudaGetLastError();
 		staged = a.type == cudaMemoryTypeUnregistered;
 	}
-	if (staged) {
-		s->pageable.run(dst, src, bytes, s->device, s->stream);
+	if (staged && s->pageable.make()) {
+		CU(s->pageable.run(dst, src, bytes, s->device, s->stream));
 	} else {
 		CU(cudaMemcpyAsync(dst, src, bytes, kind, s->stream));
 		CU(cudaStreamSynchronize(s->stream));
