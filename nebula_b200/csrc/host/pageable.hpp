@@ -8,15 +8,18 @@
 
 namespace nbl {
 
-// The driver stages such a copy through one thread (some 10 GB/s); here four
-// threads copy blocks of it into page-locked buffers and send them on from
-// there (some 18 GB/s: 92 MB of primaries 9.4 -> 5.2 ms; 128 KiB blocks 6.3,
-// 1 MiB blocks 3.6, but the larger the buffers the longer the first push takes
-// to make them).
+// The driver stages a pageable copy through one thread (10 to 12 GB/s); here
+// four threads copy blocks of it into page-locked buffers and send them on from
+// there (21 GB/s).  Making the buffers takes some 3.5 ms, which a copy has to
+// earn before it is faster than the driver's: B200, direct / first copy with
+// the buffers / later ones, in ms: 33 MB 2.2 / 4.3 / 1.7, 64 MB 4.9 / 6.3 / 3.1,
+// 80 MB 6.9 / 7.1 / 3.8, 92 MB 8.2 / 7.7 / 4.3, 256 MB 23 / 15.3 / 11.8.  (Of the
+// block sizes 128 KiB gives 6.3 ms for 92 MB and 1 MiB 3.6, but the larger the
+// buffers the longer they take to make.)
 class PageableCopy {
 public:
-	// (below, the buffers cost a simulation's first push more than they save it)
-	static constexpr size_t MIN_BYTES = (size_t)16 << 20;
+	// from here on a simulation's first copy is no slower than the driver's
+	static constexpr size_t MIN_BYTES = (size_t)80 << 20;
 	static constexpr int LANES = 4;
 	static constexpr size_t BLOCK = (size_t)256 << 10;
 

@@ -168,15 +168,15 @@ def test_reused_simulation_equals_fresh_ones(inputs):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [466_033, 466_034, 500_001])
+@pytest.mark.parametrize("n", [2_330_168, 2_330_169, 2_500_001])
 def test_large_pageable_push_equals_pinned(inputs, n):
-    """Pushes of 16 MiB and more (466 034 records) go through staging threads;
+    """Pushes of 80 MiB and more (2 330 169 records) go through staging threads;
     from page-locked memory, or in small parts, they are copied directly."""
     import torch
     from nebula_b200.synth import primaries
     g = nb.Geometry.from_tri_file(inputs["slab.tri"])
     m = nb.Material.load(inputs["si.nmat"])
-    pri = primaries.point_beam(n, energy=60.0)
+    pri = primaries.point_beam(n, energy=20.0)
     pri["px"] = np.arange(n)
     pri["pos"][:, 0] = np.random.default_rng(n).uniform(-300, 300, n)
     pinned = torch.empty(n * 36, dtype=torch.uint8, pin_memory=True).numpy().view(nb.PRI_DTYPE)
@@ -192,3 +192,24 @@ def test_large_pageable_push_equals_pinned(inputs, n):
     assert len(whole) > 0
     assert np.array_equal(_sorted(whole), _sorted(direct))
     assert np.array_equal(_sorted(whole), _sorted(parts))
+
+
+def test_first_pageable_push_waits_for_no_buffers(inputs):
+    """A first push of 24 MB takes about as long as the next one (it makes the
+    primaries' device buffer, 1.3 times).  The staging buffers, which only
+    pushes of 80 MiB and more earn back, would make it three times as long."""
+    import time
+    g = nb.Geometry.from_tri_file(inputs["slab.tri"])
+    m = nb.Material.load(inputs["si.nmat"])
+    pri = np.zeros(666_667, nb.PRI_DTYPE)
+    pri["E"] = 1.0
+    times = []
+    for _ in range(9):
+        sim = nb.Simulation(g, [m], capacity=1 << 16)
+        for _ in range(2):
+            t = time.perf_counter()
+            sim.push(pri)
+            times.append(time.perf_counter() - t)
+            sim.reset()
+        sim.close()
+    assert min(times[::2]) < 2 * min(times[1::2])
