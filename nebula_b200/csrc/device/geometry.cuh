@@ -97,6 +97,49 @@ __device__ __forceinline__ void tri_normal(const DevTriangle& T, float& nx, floa
 	nz = fs(fm(T.e1x, T.e2y), fm(T.e1y, T.e2x));
 }
 
+// A triangle's plane in units of what rounding can shift it by.
+//
+// The ray test (intersect_ray) returns t = num / det with, for a ray from s
+// along d, det = -d.n + a, num = (s - r0).n + b, where n = e1 x e2 and the
+// rounding of the two cross and dot products (u = 2^-24 per operation) gives
+// |a| <= 8 u |d| |e1| |e2| and |b| <= 10 u |s - r0| |e1| |e2|.  With H the
+// height of r0's plane over s along n, times |n|, and S = d.n, t lies in
+// (0, L] only if H sgn(S) >= -(|b| + 2 |a| L) and |H| <= L (|S| + |a|) + |b|
+// (if |S| <= |a| the sign of t is open, but then |t| > L for an |H| larger
+// than |b| + 2 |a| L).  L |d| is at most the domain's diagonal D, so both
+// allowances are at most 26 u (|s - r0| + D) |e1| |e2| / |n| as a distance;
+// evaluating the plane in float adds at most 16 u times the largest
+// coordinate.  The unit below is larger than their sum.
+__device__ __forceinline__ DevPlane plane_of(const DevTriangle& T, const DevGeometry& g)
+{
+	const double u = 1.0 / (1 << 24);
+	const double e1[3] = { T.e1x, T.e1y, T.e1z }, e2[3] = { T.e2x, T.e2y, T.e2z }, r0[3] = { T.r0x, T.r0y, T.r0z };
+	const double center[3] = { g.cx, g.cy, g.cz }, half[3] = { g.hx, g.hy, g.hz };
+	double n[3], far = 0, coord = 0, aa = 0, bb = 0, nn = 0;
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		const double reach = fabs(r0[k] - center[k]) + half[k];
+		far += reach * reach;
+		coord = fmax(coord, fmax(fabs(r0[k]), fabs(center[k]) + half[k]));
+		aa += e1[k] * e1[k];
+		bb += e2[k] * e2[k];
+	}
+#pragma unroll
+	for (int k = 0; k < 3; ++k) {
+		n[k] = e1[(k + 1) % 3] * e2[(k + 2) % 3] - e1[(k + 2) % 3] * e2[(k + 1) % 3];
+		nn += n[k] * n[k];
+	}
+	const double len = sqrt(nn);
+	const double unit = 32 * u * ((sqrt(far) + g.max_extent) * sqrt(aa * bb) / len + 2 * coord);
+	const double w = (n[0] * r0[0] + n[1] * r0[1] + n[2] * r0[2]) / len / unit;
+	DevPlane p;
+	p.x = (float)(n[0] / len / unit); p.y = (float)(n[1] / len / unit); p.z = (float)(n[2] / len / unit);
+	p.w = (float)w;
+	if (!(len > 0) || !isfinite(unit) || !isfinite(w))
+		p.x = p.y = p.z = p.w = __int_as_float(0x7fffffff);
+	return p;
+}
+
 // Whether the ray test could return a distance in (0, limit] for the triangle
 // with plane `pl`: false only when its rounded result provably lies outside,
 // because the ray meets the plane behind the start or past `limit` by more

@@ -6,8 +6,6 @@
 #include <vector>
 #include <string>
 #include <algorithm>
-#include <cmath>
-#include <limits>
 #include "internal.hpp"
 #include "../kernels.cuh"
 
@@ -65,46 +63,6 @@ inline DevTriangle device_triangle(const nbl_triangle& t)
 	return d;
 }
 
-// A triangle's plane in units of what rounding can shift it by.
-//
-// The ray test (intersect_ray) returns t = num / det with, for a ray from s
-// along d, det = -d.n + a, num = (s - r0).n + b, where n = e1 x e2 and the
-// rounding of the two cross and dot products (u = 2^-24 per operation) gives
-// |a| <= 8 u |d| |e1| |e2| and |b| <= 10 u |s - r0| |e1| |e2|.  With H the
-// height of r0's plane over s along n, times |n|, and S = d.n, t lies in
-// (0, L] only if H sgn(S) >= -(|b| + 2 |a| L) and |H| <= L (|S| + |a|) + |b|
-// (if |S| <= |a| the sign of t is open, but then |t| > L for an |H| larger
-// than |b| + 2 |a| L).  L |d| is at most the domain's diagonal D, so both
-// allowances are at most 26 u (|s - r0| + D) |e1| |e2| / |n| as a distance;
-// evaluating the plane in float adds at most 16 u times the largest
-// coordinate.  The unit below is larger than their sum.
-inline DevPlane plane_of(const nbl_triangle& t, const HostGeometry& g)
-{
-	const double u = 1.0 / (1 << 24);
-	double e1[3], e2[3], r0[3], n[3], far = 0, coord = 0, aa = 0, bb = 0, nn = 0;
-	for (int k = 0; k < 3; ++k) {
-		e1[k] = t.e1[k]; e2[k] = t.e2[k]; r0[k] = t.r0[k];
-		const double reach = std::fabs(r0[k] - g.center[k]) + g.halfsize[k];
-		far += reach * reach;
-		coord = std::max(coord, std::max(std::fabs(r0[k]), std::fabs((double)g.center[k]) + g.halfsize[k]));
-		aa += e1[k] * e1[k];
-		bb += e2[k] * e2[k];
-	}
-	for (int k = 0; k < 3; ++k) {
-		n[k] = e1[(k + 1) % 3] * e2[(k + 2) % 3] - e1[(k + 2) % 3] * e2[(k + 1) % 3];
-		nn += n[k] * n[k];
-	}
-	const double len = std::sqrt(nn);
-	const double unit = 32 * u * ((std::sqrt(far) + g.max_extent) * std::sqrt(aa * bb) / len + 2 * coord);
-	const double w = (n[0] * r0[0] + n[1] * r0[1] + n[2] * r0[2]) / len / unit;
-	DevPlane p;
-	p.x = (float)(n[0] / len / unit); p.y = (float)(n[1] / len / unit); p.z = (float)(n[2] / len / unit);
-	p.w = (float)w;
-	if (!(len > 0) || !std::isfinite(unit) || !std::isfinite(w))
-		p.x = p.y = p.z = p.w = std::numeric_limits<float>::quiet_NaN();
-	return p;
-}
-
 // Whether a mesh is fine in the sense of PASS_EMPTY: its leaves are small
 // against the flights, so that most of those crossed hold no triangle.
 inline bool fine_mesh(const HostGeometry& g) { return g.octree.size() >= (size_t)1 << 20; }
@@ -116,20 +74,14 @@ struct DeviceGeometry {
 	void upload(const HostGeometry& g, cudaStream_t s)
 	{
 		std::vector<DevTriangle> dt(g.tris.size());
-		std::vector<DevPlane> dp(g.tris.size());
-		for (size_t i = 0; i < g.tris.size(); ++i) {
+		for (size_t i = 0; i < g.tris.size(); ++i)
 			dt[i] = device_triangle(g.tris[i]);
-			dp[i] = plane_of(g.tris[i], g);
-		}
 		octree.alloc(g.octree.size() * sizeof(int32_t));
 		tris.alloc(std::max<size_t>(dt.size(), 1) * sizeof(DevTriangle));
-		planes.alloc(std::max<size_t>(dp.size(), 1) * sizeof(DevPlane));
+		planes.alloc(std::max<size_t>(dt.size(), 1) * sizeof(DevPlane));
 		CU(cudaMemcpyAsync(octree.p, g.octree.data(), g.octree.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-		if (!dt.empty()) {
+		if (!dt.empty())
 			CU(cudaMemcpyAsync(tris.p, dt.data(), dt.size() * sizeof(DevTriangle), cudaMemcpyHostToDevice, s));
-			CU(cudaMemcpyAsync(planes.p, dp.data(), dp.size() * sizeof(DevPlane), cudaMemcpyHostToDevice, s));
-		}
-		CU(cudaStreamSynchronize(s));
 		view.octree = octree.as<int32_t>();
 		view.tris = tris.as<DevTriangle>();
 		view.planes = planes.as<DevPlane>();
@@ -138,6 +90,8 @@ struct DeviceGeometry {
 		view.max_extent = g.max_extent;
 		view.n_tri = (int32_t)g.tris.size();
 		view.n_octree = (int64_t)g.octree.size();
+		CU(launch_planes(view, planes.as<DevPlane>(), s));
+		CU(cudaStreamSynchronize(s));
 	}
 };
 

@@ -148,6 +148,8 @@ struct BatchParams {
 };
 
 // launchers
+// the planes of g.tris, into `planes`
+cudaError_t launch_planes(const DevGeometry& g, DevPlane* planes, cudaStream_t s);
 cudaError_t launch_ray_query(const DevGeometry& g, const float* pos, const float* dir, const float* dist,
 	const int32_t* ignore_tri, const int32_t* ignore_mat, int64_t n, float* out_dist, int32_t* out_tri,
 	cudaStream_t s);

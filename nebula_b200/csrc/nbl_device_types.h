@@ -36,7 +36,7 @@ static_assert(sizeof(DevTriangle) == 48, "DevTriangle must be 48 bytes");
 // over a leaf's list reads only this (8 planes per cache line).  (x, y, z) is
 // the unit normal and w its product with r0, all divided by the distance the
 // ray test's float rounding can shift the triangle's plane by (plane_of in
-// host/device.hpp), so that a ray farther than 1 from the plane is past any
+// device/geometry.cuh), so that a ray farther than 1 from the plane is past any
 // rounding.  NaN for a triangle without a normal: no comparison rejects it.
 struct DevPlane { float x, y, z, w; };
 static_assert(sizeof(DevPlane) == 16, "DevPlane must be 16 bytes");

@@ -172,19 +172,13 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 		unsigned char* geom = base + OFF_GEOM;
 		cuda_ok(cudaMemcpyAsync(geom, hg.octree.data(), hg.octree.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s),
 			"copy octree");
-		unsigned char* planes = geom + oct_bytes + hg.tris.size() * sizeof(DevTriangle);
 		DevTriangle chunk[256];
-		DevPlane plane_chunk[256];
 		for (size_t i = 0; i < hg.tris.size(); i += 256) {
 			const size_t k = std::min<size_t>(256, hg.tris.size() - i);
-			for (size_t j = 0; j < k; ++j) {
+			for (size_t j = 0; j < k; ++j)
 				chunk[j] = device_triangle(hg.tris[i + j]);
-				plane_chunk[j] = plane_of(hg.tris[i + j], hg);
-			}
 			cuda_ok(cudaMemcpyAsync(geom + oct_bytes + i * sizeof(DevTriangle), chunk, k * sizeof(DevTriangle),
 				cudaMemcpyHostToDevice, s), "copy triangles");
-			cuda_ok(cudaMemcpyAsync(planes + i * sizeof(DevPlane), plane_chunk, k * sizeof(DevPlane),
-				cudaMemcpyHostToDevice, s), "copy planes");
 			cuda_ok(cudaStreamSynchronize(s), "copy triangles");
 		}
 		DevMaterial dm[NBL_NOALLOC_MAX_MATERIALS];
@@ -227,12 +221,14 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 		StepParams sp{};
 		sp.geom.octree = reinterpret_cast<const int32_t*>(geom);
 		sp.geom.tris = reinterpret_cast<const DevTriangle*>(geom + oct_bytes);
-		sp.geom.planes = reinterpret_cast<const DevPlane*>(planes);
 		sp.geom.cx = hg.center[0]; sp.geom.cy = hg.center[1]; sp.geom.cz = hg.center[2];
 		sp.geom.hx = hg.halfsize[0]; sp.geom.hy = hg.halfsize[1]; sp.geom.hz = hg.halfsize[2];
 		sp.geom.max_extent = hg.max_extent;
 		sp.geom.n_tri = (int32_t)hg.tris.size();
 		sp.geom.n_octree = (int64_t)hg.octree.size();
+		DevPlane* const planes = reinterpret_cast<DevPlane*>(geom + oct_bytes + hg.tris.size() * sizeof(DevTriangle));
+		cuda_ok(launch_planes(sp.geom, planes, s), "launch planes");
+		sp.geom.planes = planes;
 		sp.mats = reinterpret_cast<const DevMaterial*>(base + OFF_MATS);
 		sp.n_mat = n_materials;
 		sp.energy_threshold = params->energy_threshold;
