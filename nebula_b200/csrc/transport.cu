@@ -1114,7 +1114,9 @@ __device__ __forceinline__ bool grid_barrier(const BatchParams& B)
 // batch of jobs, with a grid barrier between iterations instead of a kernel
 // boundary; it ends when an iteration finds no work (all blocks see the same
 // control words) or after max_iterations (error word set).
-template<bool ADJ, uint32_t PHC = 0u>
+// FINE: 1 for a batch with a fine mesh, whose warps each go on their own and
+// whose walks pass empty leaves (batch_kernel), else 0.
+template<bool ADJ, uint32_t PHC, int FINE>
 __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepParams P,
 	const __grid_constant__ BatchParams B)
 {
@@ -1136,7 +1138,7 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 	LocalCounters lc{ s_counters, 0u };
 	uint32_t it = 0;
 	for (; it < B.max_iterations; ++it) {
-		if (!step_iteration<ADJ, true, false, PHC>(P, B, it, lc, s_mats, s_rank + (threadIdx.x & ~31u), nullptr, s_geoms, s_jobs))
+		if (!step_iteration<ADJ, true, false, PHC, FINE>(P, B, it, lc, s_mats, s_rank + (threadIdx.x & ~31u), nullptr, s_geoms, s_jobs))
 			break;
 		if (!grid_barrier(B))
 			break;
@@ -1202,14 +1204,23 @@ cudaError_t step_binary_version(int device, int* version)
 	return e;
 }
 
+// The batched kernel: the default physics selection fixed at compile time or
+// the run-time word, with a fine mesh or without.
+static const void* batch_kernel(bool fixed, bool fine)
+{
+	if (fixed)
+		return fine ? (const void*)k_batch<false, PH_DEFAULT, 1> : (const void*)k_batch<false, PH_DEFAULT, 0>;
+	return fine ? (const void*)k_batch<false, 0u, 1> : (const void*)k_batch<false, 0u, 0>;
+}
+
 int batch_grid_size(int device, int block, const StepParams& p)
 {
 	int sms = 148, per_sm = 0;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
 	// the cooperative grid must be co-resident for whichever instantiation runs
 	// (batches run without the adjoint: the host never sets it for them)
-	const void* kernels[] = { (const void*)k_batch<false>, (const void*)k_batch<false, PH_DEFAULT> };
-	for (const void* k : kernels) {
+	for (const void* k : { batch_kernel(true, false), batch_kernel(true, true), batch_kernel(false, false),
+			batch_kernel(false, true) }) {
 		int n = 0;
 		allow_shared_bytes(k, batch_shared_bytes(p));
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block, batch_shared_bytes(p));
@@ -1223,8 +1234,7 @@ cudaError_t launch_batch(const StepParams& p, const BatchParams& b, int grid, in
 	void* args[] = { const_cast<StepParams*>(&p), const_cast<BatchParams*>(&b) };
 	if (p.adjoint)
 		return cudaErrorInvalidValue;           // no batched adjoint
-	const void* k = p.phys == PH_DEFAULT ? (const void*)k_batch<false, PH_DEFAULT> : (const void*)k_batch<false>;
-	return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(block), args, batch_shared_bytes(p), s);
+	return cudaLaunchCooperativeKernel(batch_kernel(p.phys == PH_DEFAULT, p.pass_empty != 0), dim3(grid), dim3(block), args, batch_shared_bytes(p), s);
 }
 
 }  // namespace nbl

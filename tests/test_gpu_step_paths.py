@@ -102,25 +102,61 @@ def test_few_and_many_primaries_give_the_same_records(inputs, n):
     assert np.array_equal(_sorted(few), _sorted(many[many["px"] < n]))
 
 
-def test_fine_mesh_equals_batch_and_other_budgets(inputs):
-    """The batch passes no empty leaves along, the plain run on a fine mesh does."""
-    from nebula_b200.synth import geometry, primaries
-    mats = [nb.Material.load(inputs["si.nmat"]), nb.Material.load(inputs["pmma.nmat"])]
+def _rough_lines():
+    from nebula_b200.synth import geometry
     rows = geometry.rough_grating(n_lines=4, line_length=100.0, vertex_spacing=0.25)
     g = nb.Geometry.from_triangles(rows, max_depth=12, split_count=16)
     assert g.info()["n_octree"] >= 1 << 20
+    return g
+
+
+def _batch_records(geometries, mats, jobs, **kw):
+    batch = nb.Batch(geometries, mats, record_capacity=1 << 20, **{"capacity": 1 << 16, **kw})
+    batch.set_jobs(jobs)
+    batch.run()
+    rec, job = batch.records()
+    c = batch.counters()
+    batch.close()
+    return rec, job, c
+
+
+def test_fine_mesh_equals_batch_and_other_budgets(inputs):
+    """Walks on a fine mesh pass empty leaves along, in a plain run and in a
+    batch; with other budgets they pass others."""
+    from nebula_b200.synth import primaries
+    mats = [nb.Material.load(inputs["si.nmat"]), nb.Material.load(inputs["pmma.nmat"])]
+    g = _rough_lines()
     pri = primaries.raster_scan(16, 16, 20, 0.5, 300.0, 40.0, spot_sigma=1.0, seed=3)
     one, c1 = _records(g, mats, pri)
     long, c2 = _records(g, mats, pri, walk_cells=1 << 10)
-    batch = nb.Batch([g], mats, capacity=1 << 16, record_capacity=1 << 20)
-    batch.set_jobs([(0, 77, pri)])
-    batch.run()
-    rec, _ = batch.records()
-    batch.close()
+    rec, _, _ = _batch_records([g], mats, [(0, 77, pri)])
     assert c1["walk_resumes"] > 0 and c1["flights"] == c2["flights"]
     assert len(one) > 0
     assert np.array_equal(_sorted(one), _sorted(long))
     assert np.array_equal(_sorted(one), _sorted(rec))
+
+
+@pytest.mark.parametrize("physics", [None, {"interface_absorption": 1}])
+@pytest.mark.parametrize("block_size", [128, 512])
+@pytest.mark.parametrize("coarse, fine_kernel", [(0, True), (31 * 512, True), (31 * 512 + 1, False)])
+def test_batch_kernel_for_fine_meshes(inputs, physics, block_size, coarse, fine_kernel):
+    """The batched kernel for fine meshes runs from 1/32 of the primaries on.
+    Either gives the plain run's records; with it the walks on the mesh, which
+    end last here, take as many iterations as the plain run's, without it half
+    as many again (no empty leaf is passed)."""
+    from nebula_b200.synth import primaries
+    mats = [nb.Material.load(inputs["si.nmat"]), nb.Material.load(inputs["pmma.nmat"])]
+    g = _rough_lines()
+    pri = primaries.raster_scan(16, 16, 2, 0.5, 300.0, 40.0, spot_sigma=1.0, seed=3)
+    plain, c = _records(g, mats, pri, physics=physics, iterations_per_graph=6)
+    jobs = [(0, 77, pri)]
+    if coarse:
+        jobs.append((1, 77, primaries.point_beam(coarse, energy=100.0)))
+    rec, job, b = _batch_records([g, nb.Geometry.from_tri_file(inputs["slab.tri"])], mats, jobs, physics=physics,
+                                 block_size=block_size)
+    assert len(plain) > 0
+    assert np.array_equal(_sorted(plain), _sorted(rec[job == 0]))
+    assert (b["iterations"] < 1.2 * c["iterations"]) == fine_kernel
 
 
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 65])
