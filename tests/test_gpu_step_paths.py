@@ -102,12 +102,10 @@ def test_few_and_many_primaries_give_the_same_records(inputs, n):
     assert np.array_equal(_sorted(few), _sorted(many[many["px"] < n]))
 
 
-def _rough_lines():
+def _rough_lines(length=100.0, spacing=0.25):
     from nebula_b200.synth import geometry
-    rows = geometry.rough_grating(n_lines=4, line_length=100.0, vertex_spacing=0.25)
-    g = nb.Geometry.from_triangles(rows, max_depth=12, split_count=16)
-    assert g.info()["n_octree"] >= 1 << 20
-    return g
+    rows = geometry.rough_grating(n_lines=4, line_length=length, vertex_spacing=spacing)
+    return nb.Geometry.from_triangles(rows, max_depth=12, split_count=16)
 
 
 def _batch_records(geometries, mats, jobs, **kw):
@@ -126,6 +124,7 @@ def test_fine_mesh_equals_batch_and_other_budgets(inputs):
     from nebula_b200.synth import primaries
     mats = [nb.Material.load(inputs["si.nmat"]), nb.Material.load(inputs["pmma.nmat"])]
     g = _rough_lines()
+    assert g.info()["n_octree"] >= 1 << 20
     pri = primaries.raster_scan(16, 16, 20, 0.5, 300.0, 40.0, spot_sigma=1.0, seed=3)
     one, c1 = _records(g, mats, pri)
     long, c2 = _records(g, mats, pri, walk_cells=1 << 10)
@@ -157,6 +156,25 @@ def test_batch_kernel_for_fine_meshes(inputs, physics, block_size, coarse, fine_
     assert len(plain) > 0
     assert np.array_equal(_sorted(plain), _sorted(rec[job == 0]))
     assert (b["iterations"] < 1.2 * c["iterations"]) == fine_kernel
+
+
+@pytest.mark.parametrize("length, fine", [(85.0, False), (88.0, True)])
+def test_meshes_are_fine_from_half_a_million_words(inputs, length, fine):
+    """A plain run passes empty leaves on octrees of 2^19 words and more: it
+    takes fewer iterations than a batch whose coarse jobs keep the coarse
+    kernel (below, as many: up to the graph's 6 more, or 1 less, for other
+    lanes take the secondaries)."""
+    from nebula_b200.synth import primaries
+    mats = [nb.Material.load(inputs["si.nmat"]), nb.Material.load(inputs["pmma.nmat"])]
+    g = _rough_lines(length, 0.5)
+    assert (g.info()["n_octree"] >= 1 << 19) == fine
+    pri = primaries.raster_scan(16, 16, 2, 0.5, 300.0, 40.0, spot_sigma=1.0, seed=3)
+    plain, c = _records(g, mats, pri, iterations_per_graph=6)
+    rec, job, b = _batch_records([g, nb.Geometry.from_tri_file(inputs["slab.tri"])], mats,
+                                 [(0, 77, pri), (1, 77, primaries.point_beam(32 * len(pri), energy=100.0))])
+    assert len(plain) > 0
+    assert np.array_equal(_sorted(plain), _sorted(rec[job == 0]))
+    assert (c["iterations"] < b["iterations"] - 1) == fine
 
 
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 65])
