@@ -229,7 +229,7 @@ typedef struct nbl_image_filter {
 typedef struct nbl_params {
 	int32_t device;              /* CUDA device ordinal */
 	uint32_t capacity;           /* refill target: primaries are added while fewer electrons are in
-	                                flight; queues hold up to 8x this (secondaries); 0: 1 << 20 */
+	                                flight; queues hold up to 6x this (secondaries); 0: 1 << 20 */
 	float energy_threshold;      /* eV above the vacuum level, gpu_driver.h:56-59 */
 	uint64_t seed;
 	uint32_t block_size;         /* 0: 256 */

@@ -867,15 +867,13 @@ nbl_status nbl_sim_create(const nbl_geometry* g, nbl_material* const* materials,
 		sp.key.k0 = (uint32_t)params->seed;
 		sp.key.k1 = (uint32_t)(params->seed >> 32);
 		sp.capacity = cap;
-		// population bound: a cascade grows the population well past the
-		// number of primaries refilled, so every queue is sized for 8x the
-		// refill target; the secondary budget keeps the population below it
+		// Population bound, which is what the queues hold: a cascade grows the
+		// population well past the number of primaries refilled.  Since ended
+		// lanes fly most secondaries it peaks at 3.2 (slab, 1 keV) to 4.7 times
+		// the refill target (grating); pools of some tens of electrons would go
+		// to 7 or 8 times theirs and park the rest in the ring.
 		require((uint64_t)cap * 8 < (1ull << 30), "capacity too large");
-		sp.qcap = 8 * cap;
-		// secondaries are parked from 6x on: since ended lanes fly most of
-		// them, populations peak at 3.2 (slab, 1 keV) to 4.7 times the target
-		// (grating), at 7 to 8 times in pools below a hundred
-		sp.pop_bound = 6 * cap;
+		sp.qcap = 6 * cap;
 		// refill at most 1/16 of the target per iteration, so the population
 		// ramps up while the cascades of the first primaries develop
 		sp.ramp = std::max<uint32_t>(cap / 16, 256);
@@ -906,9 +904,9 @@ nbl_status nbl_sim_create(const nbl_geometry* g, nbl_material* const* materials,
 				Q.w0 = qb[6].as<float4>(); Q.w1 = qb[7].as<uint4>();
 			}
 		{
-			// overflow ring: at least twice the population bound, >= 2^20
+			// overflow ring: at least 16 times the refill target, >= 2^20
 			uint32_t ring = 1u << 20;
-			while (ring < 2 * sp.qcap) ring <<= 1;
+			while (ring < 16 * cap) ring <<= 1;
 			DevBuf* qb = s->spill;
 			qb[0].alloc((size_t)ring * sizeof(float4));
 			qb[1].alloc((size_t)ring * sizeof(float4));

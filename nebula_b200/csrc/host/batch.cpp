@@ -177,7 +177,6 @@ nbl_status nbl_batch_create(const nbl_geometry* const* geometries, int32_t n_geo
 		sp.energy_threshold = params->energy_threshold;
 		sp.capacity = cap;
 		sp.qcap = factor * cap;
-		sp.pop_bound = sp.qcap;
 		sp.ramp = std::max<uint32_t>(cap / 16, 256);
 		sp.refill_below = std::max<uint32_t>(1u, (uint32_t)((double)thr * cap));
 		sp.phys = phys;

@@ -74,8 +74,7 @@ struct StepParams {
 	float energy_threshold;
 	PhiloxKey key;
 	Queue q[2][N_QUEUES];
-	uint32_t qcap;            // queue capacity
-	uint32_t pop_bound;       // population bound (at most qcap): secondaries beyond it are parked in the ring
+	uint32_t qcap;            // queue capacity = population bound: secondaries beyond it are parked in the ring
 	uint32_t capacity;        // refill target: active electrons per iteration
 	uint32_t ramp;            // most primaries refilled per iteration
 	Queue spill;              // ring of secondaries that did not fit (power-of-two size)

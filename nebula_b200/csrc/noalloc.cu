@@ -244,7 +244,6 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 			sp.q[b][EV_WALK].w1 = reinterpret_cast<uint4*>(wb + align_up((size_t)NA_QCAP * 16));
 		}
 		sp.qcap = 8 * cap;
-		sp.pop_bound = sp.qcap;
 		sp.few = 1;                        // at most NBL_NOALLOC_MAX_CAPACITY electrons aimed at
 		sp.capacity = cap;
 		sp.ramp = std::max<uint32_t>(cap / 16, 256);

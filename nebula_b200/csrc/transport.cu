@@ -619,7 +619,7 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 	// first) ahead of new primaries while the population has room
 	const uint32_t sp_head = ld_ctrl(cr + SLOT_SPILL_HEAD);
 	const uint32_t sp_tail = ld_ctrl(cr + SLOT_SPILL_TAIL) + ld_ctrl(cr + SLOT_SPILL_PUSHED);
-	const uint32_t sp_room = active < P.pop_bound ? P.pop_bound - active : 0u;
+	const uint32_t sp_room = active < P.qcap ? P.qcap - active : 0u;
 	const uint32_t n_drain = min(sp_tail - sp_head, sp_room);
 	const uint32_t e3 = active + n_drain;
 	// no new primaries while secondaries are still parked in the ring, nor
@@ -633,12 +633,12 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 	const uint32_t nr = min(min(room, left), P.ramp);
 	const uint32_t total = e3 + nr;
 	// Secondary budget: every item leaves at most one electron in the next
-	// queues plus at most one secondary, so queueing at most pop_bound -
-	// total secondaries keeps the next population, and hence every queue,
-	// within pop_bound (at most qcap).  Secondaries beyond the budget go to the spill ring (the
+	// queues plus at most one secondary, so queueing at most qcap - total
+	// secondaries keeps the next population, and hence every queue, within
+	// qcap.  Secondaries beyond the budget go to the spill ring (the
 	// reference instead holds the parent back, PENDING in
 	// drivers/gpu/gpu_driver.inl:522-527, which can deadlock a full pool).
-	const uint32_t se_budget = P.pop_bound > total ? P.pop_bound - total : 0u;
+	const uint32_t se_budget = P.qcap > total ? P.qcap - total : 0u;
 	if (blockIdx.x == 0 && threadIdx.x == 0) {
 		cw[SLOT_CURSOR] = cursor + nr;
 		cw[SLOT_SPILL_HEAD] = sp_head + n_drain;

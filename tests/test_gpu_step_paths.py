@@ -267,3 +267,20 @@ def test_first_pageable_push_waits_for_no_buffers(inputs):
             sim.reset()
         sim.close()
     assert min(times[::2]) < 2 * min(times[1::2])
+
+
+def test_queues_hold_the_population_bound(inputs):
+    """Device memory of a simulation: queues for 6 times its capacity, the ring
+    for 16 times (52 bytes an electron, 32 more for a continued walk), records
+    for 4 times."""
+    import torch
+    g = nb.Geometry.from_tri_file(inputs["slab.tri"])
+    m = nb.Material.load(inputs["si.nmat"])
+    nb.Simulation(g, [m], capacity=1 << 10).close()      # loads the kernels
+    free = torch.cuda.mem_get_info()[0]
+    sim = nb.Simulation(g, [m], capacity=1 << 20)
+    used = free - torch.cuda.mem_get_info()[0]
+    sim.close()
+    queues = 2 * (5 * 52 + 32)
+    need = (1 << 20) * (6 * queues + 16 * 52 + 4 * 36)
+    assert need <= used < need + (1 << 20) * queues
