@@ -1,13 +1,13 @@
 """The step kernel's and the walk's variants against one another and the oracle.
 
-* Walks whose leaves hold lists longer than the 32 entries one pass of plane
-  tests covers, with slivers, grazing rays, rays in a triangle's plane and rays
-  that start outside the root cell: distance bits and triangle equal to the
-  oracle's walk, which tests every listed triangle.
+* Walks over lists of any length, those around the 32 entries one pass of plane
+  tests covers among them, with slivers, grazing rays, rays in a triangle's
+  plane and rays that start outside the root cell: distance bits and triangle
+  equal to the oracle's walk, which tests every listed triangle.
 * A run's records do not depend on which step kernel its size selects (few
   primaries or many), on the empty leaves a fine mesh's walks pass along, or on
   which lane flies a secondary.
-All comparisons are exact.
+All comparisons are exact, but for sums of doubles added in another order.
 """
 import numpy as np
 import pytest
@@ -41,13 +41,9 @@ def _triangles(n, rng):
     return np.hstack([mats, a, a + e1, a + e2])
 
 
-@pytest.mark.parametrize("n_tri", [1, 31, 32, 33, 64, 65, 300])
-def test_walk_equals_oracle_for_any_list_length(n_tri):
-    rng = np.random.default_rng(n_tri)
-    g = nb.Geometry.from_triangles(_triangles(n_tri, rng), max_depth=2, split_count=400)
-    og, tr = _oracle_geometry(g)
-    n = 200_000
-    pos = rng.uniform(-60, 60, (n, 3))
+def _rays(tr, rng, n, half):
+    """Rays of every kind through triangles in a cube of that half size."""
+    pos = rng.uniform(-1.2 * half, 1.2 * half, (n, 3))
     d = rng.standard_normal((n, 3))
     # a third of the rays start near a triangle's plane and run almost along it
     k = rng.integers(0, len(tr), n)
@@ -64,15 +60,76 @@ def test_walk_equals_oracle_for_any_list_length(n_tri):
     pos[outside] *= 30.0
     d[outside] = -pos[outside] + rng.standard_normal((outside.sum(), 3))
     d /= np.maximum(np.linalg.norm(d, axis=1, keepdims=True), 1e-30)
-    pos, d = pos.astype(np.float32), d.astype(np.float32)
-    dist = np.where(rng.random(n) < 0.5, rng.exponential(5.0, n), 1e4).astype(np.float32)
+    dist = np.where(rng.random(n) < 0.5, rng.exponential(5.0, n), 1e4)
     ignore_tri = np.where(rng.random(n) < 0.2, k, -1).astype(np.int32)
     ignore_mat = rng.choice([0, 1, -123], n).astype(np.int32)
-    gd, gt = g.ray_query(pos, d, dist, ignore_tri, ignore_mat)
-    cd, ct = og.propagate(pos, d, dist, ignore_tri, ignore_mat)
+    return pos.astype(np.float32), d.astype(np.float32), dist.astype(np.float32), ignore_tri, ignore_mat
+
+
+def _equal_to_oracle(g, og, rays):
+    gd, gt = g.ray_query(*rays)
+    cd, ct = og.propagate(*rays)
     assert np.array_equal(gt, ct), int((gt != ct).sum())
     assert np.array_equal(gd.view(np.uint32), cd.view(np.uint32))
+    return gt
+
+
+@pytest.mark.parametrize("n_tri", [1, 31, 32, 33, 64, 65, 300])
+def test_walk_equals_oracle_for_any_list_length(n_tri):
+    rng = np.random.default_rng(n_tri)
+    g = nb.Geometry.from_triangles(_triangles(n_tri, rng), max_depth=2, split_count=400)
+    og, tr = _oracle_geometry(g)
+    gt = _equal_to_oracle(g, og, _rays(tr, rng, 200_000, 50.0))
     assert n_tri < 31 or (gt >= 0).any()
+
+
+def _leaf_lists(octree):
+    """The triangle lists of an octree's leaves (child index < 0: minus the
+    start of a list, which a negative entry ends)."""
+    lists, nodes = [], [0]
+    while nodes:
+        at = nodes.pop()
+        for child in octree[at:at + 8]:
+            if child >= 0:
+                nodes.append(int(child))
+                continue
+            end = start = -int(child)
+            while octree[end] >= 0:
+                end += 1
+            lists.append(octree[start:end])
+    return lists
+
+
+@pytest.mark.parametrize("n_list", [1, 31, 32, 33, 63, 64, 65, 96, 97, 123, 124, 125])
+def test_walk_equals_oracle_around_the_passes_of_a_list(n_list):
+    """All triangles but four in one octant of the root: one leaf with a list of
+    exactly this length.  (With the four that make the root cell, the last three
+    lengths stand around a block of the kernel that makes the planes.)"""
+    rng = np.random.default_rng(1000 + n_list)
+    t = _triangles(n_list, rng)
+    t[:, 2:] = np.clip(25.0 + 0.4 * t[:, 2:], 3.0, 47.0)
+    corners = [(-50, -50, -50), (50, -40, -50), (-40, 50, -50), (-50, -40, 50)]
+    box = [[0, 1, x, y, z, x * 0.99, y, z, x, y * 0.99, z] for x, y, z in corners]
+    g = nb.Geometry.from_triangles(np.vstack([t, box]), max_depth=2, split_count=400)
+    og, tr = _oracle_geometry(g)
+    assert len(tr) == n_list + 4
+    inside = tr["r0"].min(1) > 0
+    leaf = [v for v in _leaf_lists(g.export()[0]) if np.array_equal(np.sort(v), np.flatnonzero(inside))]
+    assert len(leaf) == 1 and len(leaf[0]) == n_list
+    n = 100_000
+    pos, d, dist, ignore_tri, ignore_mat = _rays(tr, rng, n, 50.0)
+    # a fifth of the rays start inside the leaf and aim at one of its triangles
+    aim = np.arange(n) % 5 == 2
+    at = tr[rng.choice(leaf[0], n)]
+    u = rng.dirichlet([1.0, 1.0, 1.0], n)
+    target = at["r0"] + u[:, :1] * at["e1"] + u[:, 1:2] * at["e2"]
+    pos[aim] = rng.uniform(3.0, 47.0, (n, 3))[aim]
+    towards = (target - pos).astype(np.float64)
+    d[aim] = (towards / np.maximum(np.linalg.norm(towards, axis=1, keepdims=True), 1e-30))[aim]
+    dist[aim] = 1e4
+    gt = _equal_to_oracle(g, og, (pos, d, dist, ignore_tri, ignore_mat))
+    for first in range(0, n_list, 32):
+        assert np.isin(gt, leaf[0][first:first + 32]).any(), first
 
 
 def _sorted(rec):
