@@ -159,6 +159,66 @@ def test_few_and_many_primaries_give_the_same_records(inputs, n):
     assert np.array_equal(_sorted(few), _sorted(many[many["px"] < n]))
 
 
+@pytest.mark.parametrize("mesh, options", [
+    ("slab", {}), ("fine", {}),
+    ("slab", {"deposit": True}), ("fine", {"deposit": True}),
+    ("slab", {"kieft": True}), ("fine", {"kieft": True}),
+    ("fine", {"physics": {"interface_absorption": 1}}),
+    ("slab", {"adjoint": True}), ("fine", {"adjoint": True}),
+    ("slab", {"adjoint": True, "physics": {"interface_absorption": 1}}),
+    ("fine", {"adjoint": True, "deposit": True}),
+], ids=lambda v: v if isinstance(v, str) else "-".join(v) or "plain")
+def test_a_large_run_is_its_two_halves(inputs, mesh, options):
+    """2^18 + 2048 primaries take the step kernels for many electrons, the two
+    halves those for few (the adjoint on a fine mesh, or with deposits or
+    another physics selection, has one for both): the same records, images,
+    spectrum and event counts, and the same deposits and gradients but for the
+    order of their double-precision sums."""
+    from nebula_b200.synth import primaries
+    suffix = "_kieft.nmat" if options.get("kieft") else ".nmat"
+    mats = [nb.Material.load(inputs[k + suffix]) for k in ("si", "pmma")]
+    g = _rough_lines(88.0, 0.5) if mesh == "fine" else nb.Geometry.from_tri_file(inputs["slab.tri"])
+    assert (g.info()["n_octree"] >= 1 << 19) == (mesh == "fine")
+    nx, ny, per = 128, 129, 16
+    pri = primaries.raster_scan(nx, ny, per, 0.5, 100.0, 40.0 if mesh == "fine" else 5.0, spot_sigma=1.0, seed=9, pixel_streams=False)
+    half = len(pri) // 2
+    assert half <= 1 << 18 < len(pri)
+    kw = {"capacity": 1 << 17, "tally": (nx, ny), "physics": options.get("physics")}
+    if options.get("kieft"):
+        kw["physics"] = {"inelastic_model": 1}
+    if options.get("deposit"):
+        kw["deposit_grid"] = ((-50.0, -50.0, -20.0), (2.0, 2.0, 2.0), (50, 50, 25))
+    kw["adjoint"] = bool(options.get("adjoint"))
+
+    def run(part, first):
+        sim = nb.Simulation(g, mats, seed=77, **kw)
+        sim.set_primary_offset(first)
+        sim.push(part)
+        sim.run()
+        c = sim.counters()
+        se, bse, hist = sim.tallies()
+        counts = [c[k] for k in ("flights", "boundary", "elastic", "inelastic", "spawned", "detected", "terminated")]
+        sums = [sim.deposit_grid()] if options.get("deposit") else []
+        if kw["adjoint"]:
+            sums += list(sim.gradients())
+        rec = sim.flush_detected()
+        sim.close()
+        return rec, [se.astype(np.int64), bse.astype(np.int64), hist.astype(np.int64), np.array(counts)], sums
+
+    whole, parts = run(pri, 0), (run(pri[:half], 0), run(pri[half:], half))
+    assert len(whole[0]) > 1000
+    assert np.array_equal(_sorted(whole[0]), _sorted(np.concatenate([p[0] for p in parts])))
+    for w, a, b in zip(whole[1], parts[0][1], parts[1][1]):
+        assert np.array_equal(w, a + b)
+    assert all(np.abs(w).max() > 0 for w in whole[2][:1])
+    # sums of at most 10^6 doubles in any order: 10^6 * 2^-53 of the terms' sizes
+    for w, a, b in zip(whole[2], parts[0][2], parts[1][2]):
+        assert np.allclose(w, a + b, rtol=1e-9, atol=1e-9 * np.abs(w).max())
+    if kw["adjoint"]:
+        kw["adjoint"] = False
+        assert np.array_equal(_sorted(whole[0]), _sorted(run(pri, 0)[0]))
+
+
 def _rough_lines(length=100.0, spacing=0.25):
     from nebula_b200.synth import geometry
     rows = geometry.rough_grating(n_lines=4, line_length=length, vertex_spacing=spacing)
