@@ -104,10 +104,9 @@ __device__ __forceinline__ float imfp_at(const DevTable& imfp_tab, float scale, 
 }
 
 // One exponential free path: -tau * log(U), tau = 1 / (scale * exp(table(log E)))
-__device__ __forceinline__ float sample_path(const DevTable& imfp_tab, float scale, float E, float u, float& mu)
+__device__ __forceinline__ float sample_path(const DevTable& imfp_tab, float scale, float E, float u)
 {
-	mu = imfp_at(imfp_tab, scale, E);
-	const float tau = fdf(1.0f, mu);
+	const float tau = fdf(1.0f, imfp_at(imfp_tab, scale, E));
 	return fm(-tau, __logf(u));
 }
 

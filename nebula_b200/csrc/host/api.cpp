@@ -83,11 +83,17 @@ struct nbl_sim {
 	int grid = 0, block = 256;
 	int grid_for[2] = { 0, 0 };             // blocks of the step kernel for many and for few electrons
 	// Runs with at most this many primaries take the step kernel with three
-	// blocks per SM: 10 k slab primaries 1.96 against 2.27 ms, 4 001 at 15 keV
-	// 10.6 / 11.9, 50 k with deposits 3.47 / 3.80, 205 k Kieft-Bosch grating
-	// 3.95 / 4.13; at 300 k slab primaries still 10.94 / 11.17, but an adjoint
-	// scan of 410 k takes 35.3 against 34.8 and 922 k on the grating 27.0
-	// against 26.5 (four blocks second)
+	// blocks per SM.  Kernel ms with three / four blocks, primaries at 1 keV on
+	// the slab, at 500 eV on the grating, at 300 eV on the rough lines:
+	//                  25 k       100 k      200 k      262 k       400 k        1 M
+	//   slab        2.18/2.32  4.39/4.57  7.38/7.42  9.23/9.22  13.34/13.22  32.6/32.2
+	//   deposits    2.24/2.36  4.58/4.71  7.83/7.75  9.84/9.65  14.31/13.93  35.0/33.9
+	//   grating     2.01/2.18  4.37/4.46  6.99/6.87  8.62/8.43  12.28/11.89  27.9/26.8
+	//   adjoint     2.14/2.32  4.72/4.88  7.68/7.72  9.51/9.52  13.63/13.54  31.0/30.6
+	//   Kieft-Bosch 1.55/1.83  2.45/2.65  3.79/3.98  4.41/4.54   5.77/ 5.83  12.5/12.2
+	//   rough lines 4.26/4.79  7.52/7.97  11.4/11.5  14.7/14.8  21.62/21.39  43.3/41.5
+	// 2^18 is where the gains (Kieft-Bosch) and losses (grating, deposits) of
+	// 3 and 2 % even out
 	static constexpr uint64_t FEW_PRIMARIES = 1u << 18;
 	uint32_t graph_iters = 24;
 	uint64_t iteration = 0;
@@ -179,7 +185,7 @@ struct nbl_sim {
 
 	// A graph holds the step kernel's parameters and grid by value, so it
 	// serves every run with the same ones: capturing and instantiating its 24
-	// launches again on each push takes some 0.1 ms.
+	// launches again on each push takes 0.2 to 0.3 ms.
 	void build_graph()
 	{
 		sp.few = n_pri <= FEW_PRIMARIES ? 1 : 0;

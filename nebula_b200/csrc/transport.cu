@@ -379,10 +379,10 @@ __device__ __forceinline__ void flight_sample(const RunView& rv, const Electron&
 		const DevMaterial* const m = mats + mat;
 		PhiloxStream r;
 		r.init(rv.key, event, 0u, stream_tag, lineage);
-		float u[4], mu;
+		float u[4];
 		r.block(0, u);
-		const float pe = sample_path(m->el_imfp, m->el_scale, p.E, u[0], mu);
-		const float pi = sample_path(m->in_imfp, m->in_scale, p.E, u[1], mu);
+		const float pe = sample_path(m->el_imfp, m->el_scale, p.E, u[0]);
+		const float pi = sample_path(m->in_imfp, m->in_scale, p.E, u[1]);
 		fr.dist = __int_as_float(0x7f800000);
 		if (pe < fr.dist) { fr.dist = pe; fr.type = 2; }
 		if (pi < fr.dist) { fr.dist = pi; fr.type = 1; }
@@ -415,7 +415,10 @@ __device__ __forceinline__ int flight_walk(const StepParams& P, const RunView& r
 		// score of the flight: density mu_k exp(-(mu_in+mu_el) d) of the
 		// chosen event k at distance d, or survival exp(-(mu_in+mu_el) d)
 		// when a boundary cuts the flight; derivative w.r.t. the scales
-		// (the inverse mean free paths are those it was sampled with)
+		// (the inverse mean free paths are those it was sampled with, looked up
+		// again: kept in registers from there the replay of 160 x 160 x 100
+		// grating primaries takes 75.2 instead of 75.7 ms, the one on the rough
+		// lines 28.6 instead of 28.4)
 		const DevMaterial* const m = mats + mat;
 		const float mu_el = imfp_at(m->el_imfp, m->el_scale, p.E);
 		const float mu_in = imfp_at(m->in_imfp, m->in_scale, p.E);
@@ -665,13 +668,15 @@ __device__ __forceinline__ bool step_iteration(const StepParams& P, const BatchP
 	// claims one item per thread and its warps go through a chunk's phases
 	// (state, event, sampling, walk, append) together: the phases' code is 74 KB,
 	// far more than the instruction caches next to the schedulers, and warps
-	// that stand in the same phase fetch it once.  That takes the stalls for
-	// instructions from 3.0 to 0.5 per issued one for less than that in waits
-	// at the barriers: grating 160 x 160 x 100 68.2 -> 65.8 ms, slab 300 k 11.0
-	// -> 10.4, 10 k 2.05 -> 1.82, batch of 20 jobs 23.7 -> 21.5; blocks of 128
+	// that stand in the same phase fetch it once.  In a full iteration on the
+	// grating that takes the stalls for instructions from 3.4 to 0.6 per issued
+	// one, for 2.2 instead of 0.2 in waits at the barriers, and 312 to 289 us:
+	// grating 160 x 160 x 100 68.2 -> 65.8 ms, slab 300 k 11.0 -> 10.4, 10 k
+	// 2.05 -> 1.82, batch of 20 jobs 23.7 -> 21.5; blocks of 128
 	// and 512 threads gain less.  On a fine mesh, whose walks wait for loads of
 	// very different latency, the barriers cost more than they save (64.3 ->
-	// 65.2 ms on the rough lines): there each warp claims its own chunk.
+	// 65.2 ms on the rough lines, a batch on them 96 -> 124 with the empty
+	// leaves): there each warp claims its own chunk.
 	constexpr bool TOGETHER = FINE != 1;
 	const auto phase = [] { if (TOGETHER) __syncthreads(); };
 	uint32_t* const work = P.ctrl + rs * SLOT_WORDS + SLOT_WORK;
@@ -1051,11 +1056,16 @@ __device__ __forceinline__ void flush_counters(const StepParams& P, LocalCounter
 // none of their code).  PHC: nonzero = the physics selection fixed at
 // compile time (PH_DEFAULT only).  FINE: a fine mesh (1), a coarse one (0), or
 // what P.pass_empty says (-1).
+// The run-time variants take the phases together on fine meshes too; they were
+// faster there than the kernels before the phases (553 k primaries on the rough
+// lines: deposits 28.4 -> 27.1 ms, Kieft-Bosch 16.8 -> 14.8), and an
+// instantiation more would gain the 1 % that warps on their own do.
 // BLOCKS: resident blocks of 256 threads per SM.  Four (64 registers a thread,
 // some spilled) where the chip is full: the kernel waits for loads and
 // instruction fetches, and warps in flight matter more than the spills.  Three
-// (80 registers, none spilled) for runs that never fill it, whose time is the
-// latency of one chunk after the other.
+// (80 registers, none spilled; the adjoint 44 bytes) for runs of few primaries,
+// most of whose iterations hold less than one chunk for each warp: their time is
+// the latency of one chunk after the other (FEW_PRIMARIES in host/api.cpp).
 template<bool ADJ, bool DEP, uint32_t PHC, int FINE, int BLOCKS>
 __global__ void __launch_bounds__(256, BLOCKS) k_step(const __grid_constant__ StepParams P, uint32_t it)
 {
@@ -1153,7 +1163,9 @@ __global__ void __launch_bounds__(512, 2) k_batch(const __grid_constant__ StepPa
 
 // The step kernel instantiation a run's parameters select: adjoint or not,
 // deposits or not, the default physics selection fixed at compile time or the
-// run-time word, fine or coarse mesh, few electrons or many.
+// run-time word, fine or coarse mesh, few electrons or many.  The adjoint on a
+// fine mesh, with deposits or with another selection has the one of four blocks
+// for both (not timed with three).
 template<bool ADJ, bool DEP, uint32_t PHC, int FINE>
 static const void* step_kernel_for(const StepParams& p)
 {
