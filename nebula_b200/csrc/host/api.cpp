@@ -293,6 +293,7 @@ struct nbl_sim {
 		}
 		for (uint64_t k = 0; k < max_graphs; ++k) {
 			launch_graph();
+			pageable.make_wanted();             // while the device is busy
 			if (sink_pending) {
 				sink_copy(sink_upto);
 				sink_pending = false;
@@ -1033,7 +1034,7 @@ static void push_common(nbl_sim* s, const void* src, int64_t n, cudaMemcpyKind k
 			cudaGetLastError();
 		staged = a.type == cudaMemoryTypeUnregistered;
 	}
-	if (staged && s->pageable.make()) {
+	if (staged && s->pageable.takes(bytes)) {
 		CU(s->pageable.run(dst, src, bytes, s->device, s->stream));
 	} else {
 		CU(cudaMemcpyAsync(dst, src, bytes, kind, s->stream));

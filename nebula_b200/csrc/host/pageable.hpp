@@ -10,16 +10,21 @@ namespace nbl {
 
 // The driver stages a pageable copy through one thread (10 to 12 GB/s); here
 // four threads copy blocks of it into page-locked buffers and send them on from
-// there (21 GB/s).  Making the buffers takes some 3.5 ms, which a copy has to
-// earn before it is faster than the driver's: B200, direct / first copy with
-// the buffers / later ones, in ms: 33 MB 2.2 / 4.3 / 1.7, 64 MB 4.9 / 6.3 / 3.1,
-// 80 MB 6.9 / 7.1 / 3.8, 92 MB 8.2 / 7.7 / 4.3, 256 MB 23 / 15.3 / 11.8.  (Of the
-// block sizes 128 KiB gives 6.3 ms for 92 MB and 1 MiB 3.6, but the larger the
-// buffers the longer they take to make.)
+// there (21 GB/s).  Making the buffers takes some 3 ms, which a copy has to earn
+// before it is faster than the driver's: B200, direct / first copy with the
+// buffers made for it / later ones, in ms: 33 MB 2.2 / 4.3 / 1.7, 48 MB
+// 3.4 / 5.6 / 2.3, 64 MB 4.9 / 6.3 / 3.1, 80 MB 6.9 / 7.1 / 3.8, 92 MB
+// 8.2 / 7.7 / 4.3, 256 MB 23 / 15.3 / 11.8.  So a copy of FIRST_BYTES makes the
+// buffers at once.  Of those from MIN_BYTES on the first two are the driver's:
+// an object that copies a second time is likely to go on, and the buffers are
+// made where the host next waits for the device (nbl_sim::advance).  (Of
+// the block sizes 128 KiB gives 5.8 ms for 92 MB and 64 KiB 8.6: each block's
+// copy takes 8 us to issue.  1 MiB gives 3.6, but the larger the buffers the
+// longer they take to make.)
 class PageableCopy {
 public:
-	// from here on a simulation's first copy is no slower than the driver's
-	static constexpr size_t MIN_BYTES = (size_t)80 << 20;
+	static constexpr size_t MIN_BYTES = (size_t)40 << 20;
+	static constexpr size_t FIRST_BYTES = (size_t)80 << 20;
 	static constexpr int LANES = 4;
 	static constexpr size_t BLOCK = (size_t)256 << 10;
 
@@ -34,8 +39,28 @@ public:
 		if (buffer) cudaFreeHost(buffer);
 	}
 
-	// Makes the buffers, once.  False where that is not possible: such a copy
-	// is the driver's, which needs none of them.
+	// Whether this copy of pageable memory should go through run().  False: it
+	// is the driver's, which needs no buffers.
+	bool takes(size_t bytes)
+	{
+		if (bytes < MIN_BYTES)
+			return false;
+		if (!ready && bytes >= FIRST_BYTES)
+			make();
+		wanted = again && !ready;
+		again = true;
+		return ready;
+	}
+
+	// Makes the buffers if a copy would have liked them.
+	void make_wanted()
+	{
+		if (wanted)
+			make();
+		wanted = false;
+	}
+
+	// Makes the buffers, once.  False where that is not possible.
 	bool make()
 	{
 		bool made = buffer || cudaHostAlloc((void**)&buffer, 2 * LANES * BLOCK, cudaHostAllocDefault) == cudaSuccess;
@@ -44,11 +69,12 @@ public:
 				made = made && (e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess);
 		if (!made)
 			cudaGetLastError();
+		ready = made;
 		return made;
 	}
 
 	// Enqueues on `stream` (of the current device, `device`) and returns when
-	// all of it has arrived.  make() has returned true before.
+	// all of it has arrived.  make() or takes() has returned true before.
 	cudaError_t run(void* dst, const void* src, size_t bytes, int device, cudaStream_t stream)
 	{
 		const auto part = [=](int lane) { work(lane, dst, src, bytes, device, stream); };
@@ -80,6 +106,9 @@ private:
 	};
 	Lane lanes[LANES];
 	char* buffer = nullptr;       // 2 MiB
+	bool ready = false;           // it and the events are made
+	bool again = false;           // there was a copy of MIN_BYTES
+	bool wanted = false;          // there was another, without the buffers
 
 	// blocks lane, lane + LANES, ... through the lane's two buffers in turn
 	void work(int lane, void* dst, const void* src, size_t bytes, int device, cudaStream_t stream) noexcept

@@ -339,10 +339,11 @@ def test_reused_simulation_equals_fresh_ones(inputs):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [2_330_168, 2_330_169, 2_500_001])
+@pytest.mark.parametrize("n", [1_165_084, 1_165_085, 2_330_168, 2_330_169, 2_500_001])
 def test_large_pageable_push_equals_pinned(inputs, n):
-    """Pushes of 80 MiB and more (2 330 169 records) go through staging threads;
-    from page-locked memory, or in small parts, they are copied directly."""
+    """Pushes of 80 MiB and more (2 330 169 records) go through staging threads,
+    those of 40 MiB and more (1 165 085) from a simulation's third run on; from
+    page-locked memory, or in small parts, they are copied directly."""
     import torch
     from nebula_b200.synth import primaries
     g = nb.Geometry.from_tri_file(inputs["slab.tri"])
@@ -352,27 +353,27 @@ def test_large_pageable_push_equals_pinned(inputs, n):
     pri["pos"][:, 0] = np.random.default_rng(n).uniform(-300, 300, n)
     pinned = torch.empty(n * 36, dtype=torch.uint8, pin_memory=True).numpy().view(nb.PRI_DTYPE)
     pinned[:] = pri
-    whole, _ = _records(g, [m], pri, capacity=1 << 16)
     direct, _ = _records(g, [m], pinned, capacity=1 << 16)
     sim = nb.Simulation(g, [m], capacity=1 << 16, seed=77)
-    for part in np.array_split(pri, 5):
-        sim.push(part)
-    sim.run()
-    parts = sim.flush_detected()
+    for parts in (1, 1, 1, 9):
+        for part in np.array_split(pri, parts):
+            sim.push(part)
+        sim.run()
+        rec = sim.flush_detected()
+        sim.reset()
+        assert len(rec) > 0
+        assert np.array_equal(_sorted(rec), _sorted(direct)), parts
     sim.close()
-    assert len(whole) > 0
-    assert np.array_equal(_sorted(whole), _sorted(direct))
-    assert np.array_equal(_sorted(whole), _sorted(parts))
 
 
 def test_first_pageable_push_waits_for_no_buffers(inputs):
     """A first push of 24 MB takes about as long as the next one (it makes the
-    primaries' device buffer, 1.3 times).  The staging buffers, which only
-    pushes of 80 MiB and more earn back, would make it three times as long."""
+    primaries' device buffer, 1.3 times).  Making the staging buffers for it
+    would take three times as long."""
     import time
     g = nb.Geometry.from_tri_file(inputs["slab.tri"])
     m = nb.Material.load(inputs["si.nmat"])
-    pri = np.zeros(666_667, nb.PRI_DTYPE)
+    pri = np.zeros(24_000_000 // 36, nb.PRI_DTYPE)
     pri["E"] = 1.0
     times = []
     for _ in range(9):

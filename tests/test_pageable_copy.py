@@ -86,6 +86,15 @@ int main(int argc, char** argv)
 			fail = "";
 			if (!c.make()) return 4;
 		}
+		nbl::PageableCopy d;                          // a copy of FIRST_BYTES makes the buffers
+		if (d.takes(c.MIN_BYTES - 1) || d.takes(c.MIN_BYTES - 1)) return 9;
+		if (!d.takes(c.FIRST_BYTES) || !d.takes(c.MIN_BYTES) || d.takes(c.MIN_BYTES - 1)) return 10;
+		nbl::PageableCopy w;                          // of smaller ones the second asks for them
+		for (int k = 0; k < 2; ++k) {
+			if (w.make_wanted(), w.takes(c.MIN_BYTES)) return 11;
+			if (w.takes(c.MIN_BYTES - 1)) return 12;
+		}
+		if (w.make_wanted(), !w.takes(c.MIN_BYTES)) return 13;
 		// the second helper thread finds no memory, after the first has started
 		if (fail == "memory") countdown = 1;
 		const cudaError_t e = c.run(dst.data(), src.data(), n, 0, nullptr);
