@@ -8,22 +8,22 @@
 
 namespace nbl {
 
-// The driver stages a pageable copy through one thread (10 to 12 GB/s); here
-// four threads copy blocks of it into page-locked buffers and send them on from
-// there (21 GB/s).  Making the buffers takes some 3 ms, which a copy has to earn
-// before it is faster than the driver's: B200, direct / first copy with the
-// buffers made for it / later ones, in ms: 33 MB 2.2 / 4.3 / 1.7, 48 MB
-// 3.4 / 5.6 / 2.3, 64 MB 4.9 / 6.3 / 3.1, 80 MB 6.9 / 7.1 / 3.8, 92 MB
-// 8.2 / 7.7 / 4.3, 256 MB 23 / 15.3 / 11.8.  So a copy of FIRST_BYTES makes the
-// buffers at once.  Of those from MIN_BYTES on the first two are the driver's:
-// an object that copies a second time is likely to go on, and the buffers are
-// made where the host next waits for the device (nbl_sim::advance).  (Of
-// the block sizes 128 KiB gives 5.8 ms for 92 MB and 64 KiB 8.6: each block's
-// copy takes 8 us to issue.  1 MiB gives 3.6, but the larger the buffers the
-// longer they take to make.)
+// The driver stages a pageable copy through one thread (10 to 12 GB/s); here four
+// threads copy blocks of it into page-locked buffers and send them on from there
+// (21 GB/s).  Making the buffers takes some 3 ms, which a copy has to earn before
+// it is faster than the driver's: B200, direct / first copy with the buffers made
+// for it / later ones, in ms: 17 MB 1.2 / 3.5 / 1.0, 25 MB 1.7 / 3.7 / 1.35, 33
+// MB 2.3 / 4.3 / 1.8, 48 MB 3.4 / 5.6 / 2.4, 64 MB 4.9 / 6.3 / 3.1, 80 MB 6.9 /
+// 7.1 / 3.8, 92 MB 7.9 / 7.7 / 4.4, 256 MB 23 / 15.3 / 11.8.  So a copy of
+// FIRST_BYTES makes the buffers at once.  Of those from MIN_BYTES on the first
+// two are the driver's: an object that copies a second time is likely to go on,
+// and the buffers are made where the host next waits for the device
+// (nbl_sim::advance).  (Of the block sizes 128 KiB gives 5.8 ms for 92 MB and 64
+// KiB 8.6: each block's copy takes 8 us to issue.  1 MiB gives 3.6, but the
+// larger the buffers the longer they take to make.)
 class PageableCopy {
 public:
-	static constexpr size_t MIN_BYTES = (size_t)40 << 20;
+	static constexpr size_t MIN_BYTES = (size_t)24 << 20;
 	static constexpr size_t FIRST_BYTES = (size_t)80 << 20;
 	static constexpr int LANES = 4;
 	static constexpr size_t BLOCK = (size_t)256 << 10;

@@ -339,10 +339,10 @@ def test_reused_simulation_equals_fresh_ones(inputs):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [1_165_084, 1_165_085, 2_330_168, 2_330_169, 2_500_001])
+@pytest.mark.parametrize("n", [699_050, 699_051, 2_330_168, 2_330_169, 2_500_001])
 def test_large_pageable_push_equals_pinned(inputs, n):
     """Pushes of 80 MiB and more (2 330 169 records) go through staging threads,
-    those of 40 MiB and more (1 165 085) from a simulation's third run on; from
+    those of 24 MiB and more (699 051) from a simulation's third run on; from
     page-locked memory, or in small parts, they are copied directly."""
     import torch
     from nebula_b200.synth import primaries
