@@ -51,17 +51,19 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "primaries/s on 1 B200, plain vs batched; adjoint:forward time at yield err ≤3σ"
-BYTES_PER_EVENT = 96   # 48-byte electron state read + written per event
+# the algorithmic bytes: a 48-byte electron state read and written per event.
+# The kernel moves less state than that, for 0.61 of its flights end in a queued
+# event (52 bytes) and 0.22 in a walk that continues (84)
+BYTES_PER_EVENT = 96
 # DRAM bytes (read + write) per event of the transport kernel, measured on a
 # bounded case of this workload: the same grating scan at a pool of 2^20
-# (4.8 GB on the device), one whole graph of 6 launches in the middle of the
+# (4.7 GB on the device), one whole graph of 6 launches in the middle of the
 # scan (launches 240-245, two ncu captures of 3 launches, warm L2:
 # --cache-control none), dram__bytes_read.sum + dram__bytes_write.sum over
-# those launches / the free flights of that graph (--trace-graphs).  It
-# exceeds the 96 algorithmic bytes because a flight whose walk continues in
-# the next iteration reads and writes its state again, plus 32 bytes of walk
-# state each way.
-DRAM_BYTES_PER_EVENT = 113.1
+# those launches / the free flights of that graph (--trace-graphs): the queued
+# events and continued walks above and some 0.1 queued secondaries per flight,
+# each way; records, primaries and partial sectors are the rest.
+DRAM_BYTES_PER_EVENT = 113.0
 
 
 def measured_peaks():
