@@ -245,6 +245,7 @@ extern "C" nbl_status nbl_run_noalloc(const nbl_geometry* g, nbl_material* const
 		}
 		sp.qcap = 8 * cap;
 		sp.few = 1;                        // at most NBL_NOALLOC_MAX_CAPACITY electrons aimed at
+		// (pass_empty stays 0: no octree within NA_GEOM_BYTES has the words of a fine mesh)
 		sp.capacity = cap;
 		sp.ramp = std::max<uint32_t>(cap / 16, 256);
 		sp.refill_below = cap;
